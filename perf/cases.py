@@ -35,24 +35,24 @@ def _step(name, model, decoders=0, context=0, portion=0, past=0, ragged=False, d
 def listed():
     return [
         # one user's chat: a token at a time, where the launches and the latency of every kernel count
-        _step("decode 1, 0.6b", "0.6b", decoders=1, context=700),
+        _step("decode 1 0.6b", "0.6b", decoders=1, context=700),
         # the headline of bench.py: eight requests with contexts of 2048 tokens
-        _step("decode 8, 0.6b", "0.6b", decoders=8, context=2048),
+        _step("decode 8 0.6b", "0.6b", decoders=8, context=2048),
         # a busy server at the larger size: requests of all ages
-        _step("decode 64 ragged, 1.7b", "1.7b", decoders=64, context=2304, ragged=True),
+        _step("decode 64 ragged 1.7b", "1.7b", decoders=64, context=2304, ragged=True),
         # a long prompt in one step
-        _step("prompt 2048, 0.6b", "0.6b", portion=2048),
+        _step("prompt 2048 0.6b", "0.6b", portion=2048),
         # a question of a sentence or two: the time to its first token
-        _step("prompt 129, 0.6b", "0.6b", portion=129),
+        _step("prompt 129 0.6b", "0.6b", portion=129),
         # continuous batching under a budget of 512 rows: a portion of a prompt beside the others' decode tokens
-        _step("mixed 512, 1.7b", "1.7b", decoders=31, context=1500, ragged=True, portion=481, past=512),
+        _step("mixed 512 1.7b", "1.7b", decoders=31, context=1500, ragged=True, portion=481, past=512),
         # the true 32-bit path, with which a user checks what the 16-bit one says
-        _step("prompt 200, 0.6b f32", "0.6b", portion=200, dtype="f32"),
+        _step("prompt 200 0.6b f32", "0.6b", portion=200, dtype="f32"),
         # the other designs: a prompt, and a decode step of a small batch
-        _step("prompt 2048, sagelorn", "sagelorn", portion=2048),
-        _step("decode 8, sagelorn", "sagelorn", decoders=8, context=1500),
-        _step("prompt 1531, kedavik", "kedavik", portion=1531),
-        _step("decode 16, kedavik", "kedavik", decoders=16, context=900),
+        _step("prompt 2048 sagelorn", "sagelorn", portion=2048),
+        _step("decode 8 sagelorn", "sagelorn", decoders=8, context=1500),
+        _step("prompt 1531 kedavik", "kedavik", portion=1531),
+        _step("decode 16 kedavik", "kedavik", decoders=16, context=900),
         # a token for every row of a batch of 32: greedy, temperature, top-k and top-p side by side
         {"name": "sample 32", "kind": "sample", "rows": 32, "vocab": VOCAB},
     ]

@@ -122,6 +122,16 @@ class PageList:
         return self.arr[:self.n]
 
 
+class SavedStates:
+    """A request's state slots as they were before a step: row ``row`` of ``copies`` (a state tensor's entry -> the
+    copies of all of that step's requests)."""
+
+    __slots__ = ("copies", "row")
+
+    def __init__(self, copies: Dict[int, torch.Tensor], row: int):
+        self.copies, self.row = copies, row
+
+
 @dataclass
 class RequestCache:
     rid: Hashable
@@ -130,8 +140,8 @@ class RequestCache:
     pending: int = 0                                  # tokens appended, not yet committed
     confirmed_tokens: int = 0                         # length whose steps were seen to succeed (<= num_tokens)
     unconfirmed: List[int] = field(default_factory=list)   # token counts of committed steps not yet confirmed, oldest first
-    state_before: List[Dict[int, torch.Tensor]] = field(default_factory=list)   # state slot before each of those steps
-    state_pending: Optional[Dict[int, torch.Tensor]] = None   # ... and before the step being appended
+    state_before: List["SavedStates"] = field(default_factory=list)   # state slot before each of those steps
+    state_pending: Optional["SavedStates"] = None     # ... and before the step being appended
     pages: List[PageList] = field(default_factory=list)    # per group: page id per page index, -1 = given back
     first_live: List[int] = field(default_factory=list)    # per group: first page index still held
 
@@ -204,6 +214,9 @@ class CacheManager:
                 grp.kv = torch.zeros((len(grp.entries),) + shape, dtype=dtype, device=device)
         self.slots = StateSlotPool(max_requests)
         self.requests: Dict[Hashable, RequestCache] = {}
+        # copies rows of several tensors in one launch (the kernel pack's ``copy_state_slots``); None: tensor by tensor
+        self.slot_copier = None
+        self._slots_in_words = all(t[0].numel() * t.element_size() % 4 == 0 for t in self.state_tensors.values())
 
     # -- sizes ----------------------------------------------------------------
     def bytes_per_token(self) -> int:
@@ -217,9 +230,48 @@ class CacheManager:
         slot = self.slots.acquire(rid)
         rc = RequestCache(rid, slot, pages=[PageList() for _ in self.groups], first_live=[0 for _ in self.groups])
         self.requests[rid] = rc
+        self._clear_slot(slot)
+        return rc
+
+    # -- state slots ------------------------------------------------------------
+    @property
+    def _copier(self):
+        return self.slot_copier if self._slots_in_words else None       # (it moves whole 32-bit words)
+
+    def _clear_slot(self, slot: int) -> None:
+        if self._copier is not None and self.state_tensors:
+            self._copier([(slot, 0)], [(t, None) for t in self.state_tensors.values()])
+            return
         for t in self.state_tensors.values():
             t[slot].zero_()
-        return rc
+
+    def _save_slots(self, reqs: Sequence[RequestCache], index: Optional[torch.Tensor] = None) -> None:
+        """Queue a copy of these requests' state slots and note it as what stood before the step being appended.
+        ``index``: their slots, on the device."""
+        if self._copier is not None:
+            copies = {e: t.new_empty((len(reqs),) + tuple(t.shape[1:])) for e, t in self.state_tensors.items()}
+            self._copier([(i, rc.slot) for i, rc in enumerate(reqs)],
+                             [(copies[e], t) for e, t in self.state_tensors.items()])
+        else:
+            if index is None:
+                index = torch.tensor([rc.slot for rc in reqs], dtype=torch.int32, device=self.device)
+            copies = {e: t.index_select(0, index) for e, t in self.state_tensors.items()}
+        for i, rc in enumerate(reqs):
+            rc.state_pending = SavedStates(copies, i)
+
+    def _restore_slots(self, saved: Sequence[Tuple[int, SavedStates]]) -> None:
+        """Queue the copies back into their slots: one launch for all requests that were saved together."""
+        if self._copier is None:
+            for slot, s in saved:
+                for e, t in s.copies.items():
+                    self.state_tensors[e][slot].copy_(t[s.row])
+            return
+        together: Dict[int, List[Tuple[int, SavedStates]]] = {}
+        for slot, s in saved:
+            together.setdefault(id(s.copies), []).append((slot, s))
+        for group in together.values():
+            copies = group[0][1].copies
+            self._copier([(slot, s.row) for slot, s in group], [(self.state_tensors[e], t) for e, t in copies.items()])
 
     def has_request(self, rid: Hashable) -> bool:
         return rid in self.requests
@@ -262,32 +314,42 @@ class CacheManager:
             rc.pages[g].extend(self.groups[g].pool.allocate(c, rid))
         if snapshot and rc.pending == 0 and self.state_tensors:
             # the state as it is before this step (copies queued on the current stream, ahead of the step)
-            rc.state_pending = {e: t[rc.slot].clone() for e, t in self.state_tensors.items()}
+            self._save_slots([rc])
         rc.pending += n_new
 
     def snapshot_states(self, rids: Sequence[Hashable], slots: torch.Tensor) -> None:
-        """The state slots of the step's requests as they are before the step, for ``rollback``: ONE gather a state
-        tensor for all requests (``slots``: their slots in the order of ``rids``, int32 on the device — the step's own
-        array), instead of a copy a request and tensor, which for eight requests and eight layers with a state was
-        64 launches a step.  Queued on the current stream, ahead of the step."""
+        """The state slots of the step's requests as they are before the step, for ``rollback``: one copy of all of them
+        (``slots``: their slots in the order of ``rids``, int32 on the device — the step's own array), instead of a copy
+        a request and tensor, which for eight requests and eight layers with a state was 64 launches a step.  Queued on
+        the current stream, ahead of the step."""
         if not self.state_tensors:
             return
         reqs = [self.requests[r] for r in rids]
         if any(rc.state_pending is not None for rc in reqs):           # (a second append before a commit: one by one)
             for rc in reqs:
                 if rc.state_pending is None:
-                    rc.state_pending = {e: t[rc.slot].clone() for e, t in self.state_tensors.items()}
+                    self._save_slots([rc])
             return
-        index = slots[:len(reqs)]
-        saved = {e: t.index_select(0, index) for e, t in self.state_tensors.items()}
-        for i, rc in enumerate(reqs):
-            rc.state_pending = {e: rows[i] for e, rows in saved.items()}
+        self._save_slots(reqs, slots[:len(reqs)])
 
     def rollback(self, rid: Hashable, unconfirmed: bool = False) -> None:
         """Undo appends that were not committed (the step did not run): their pages go back, and the state
         slot is as it was before the step.  With ``unconfirmed`` also the committed steps that were not
         confirmed: the request returns to its confirmed length, pages and state."""
-        rc = self.requests[rid]
+        self.rollback_all([rid], unconfirmed)
+
+    def rollback_all(self, rids: Sequence[Hashable], unconfirmed: bool = False) -> None:
+        """``rollback`` of several requests; the state slots that one step saved go back in one launch."""
+        saved = []
+        for rid in rids:
+            rc = self.requests[rid]
+            states = self._roll_back(rc, unconfirmed)
+            if states is not None:
+                saved.append((rc.slot, states))
+        if saved:
+            self._restore_slots(saved)
+
+    def _roll_back(self, rc: RequestCache, unconfirmed: bool) -> Optional[SavedStates]:
         saved = rc.state_pending
         if unconfirmed:
             if rc.state_before:
@@ -297,12 +359,10 @@ class CacheManager:
             rc.state_before.clear()
         keep = -(-rc.num_tokens // self.page_size)
         for g, grp in enumerate(self.groups):
-            grp.pool.free([p for p in rc.pages[g].truncate(keep) if p >= 0], rid)
-        if saved is not None:
-            for e, t in saved.items():
-                self.state_tensors[e][rc.slot].copy_(t)
+            grp.pool.free([p for p in rc.pages[g].truncate(keep) if p >= 0], rc.rid)
         rc.pending = 0
         rc.state_pending = None
+        return saved
 
     def commit(self, rid: Hashable, confirmed: bool = True) -> None:
         """The step was run (``confirmed``) or queued on the device (not ``confirmed``): the appended tokens
@@ -361,8 +421,7 @@ class CacheManager:
         rc.unconfirmed.clear()
         rc.state_before.clear()
         rc.state_pending = None
-        for t in self.state_tensors.values():
-            t[rc.slot].zero_()
+        self._clear_slot(rc.slot)
 
     def num_free_pages(self) -> List[int]:
         return [g.pool.num_free for g in self.groups]

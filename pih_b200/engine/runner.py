@@ -97,6 +97,7 @@ class ModelRunner:
         self.model = model
         self.cache = cache
         self.device = model.rt.device
+        cache.slot_copier = getattr(model.rt.ops, "copy_state_slots", None)
         self.builder = BatchBuilder(self.device)
         self.num_entries = len(model.cache_needs())      # the schedule's entries and what the model itself keeps
         self.steps_run = 0
@@ -171,9 +172,7 @@ class ModelRunner:
 
     def discard(self, rids) -> None:
         """A queued step of these requests failed: they return to their confirmed length, pages and state."""
-        for rid in rids:
-            if self.cache.has_request(rid):
-                self.cache.rollback(rid, unconfirmed=True)
+        self.cache.rollback_all([rid for rid in rids if self.cache.has_request(rid)], unconfirmed=True)
 
     def _commit(self, rid) -> None:
         self.cache.commit(rid, confirmed=self._confirm)

@@ -113,7 +113,7 @@ class CudaOps:
                      "pih_act_mul", "pih_embed_positions", "pih_hyper_stream", "pih_window_qk_prepare",
                      "pih_window_attention", "pih_window_attention_tile_takes", "pih_embed_bigram", "pih_rmsnorm_rows",
                      "pih_rotate_heads", "pih_gate_mul", "pih_unary_act", "pih_selective_scan", "pih_gemm_skinny_bias_gelu", "pih_scale_rows", "pih_moe_gather_scaled",
-                     "pih_softcap_rows", "pih_stream_norm_norm", "pih_gated_part_rmsnorm", "pih_linear_memory", "pih_memory_copies"):
+                     "pih_softcap_rows", "pih_stream_norm_norm", "pih_gated_part_rmsnorm", "pih_linear_memory", "pih_memory_copies", "pih_copy_slots"):
             getattr(lib, name).restype = c_int
         lib.pih_attention_scratch_floats.restype = c_ll
         lib.pih_top_logprobs_scratch_words.restype = c_ll
@@ -196,6 +196,17 @@ class CudaOps:
         return c_void_p(self._error.data_ptr())
 
     # -- ops ----------------------------------------------------------------------
+    def copy_state_slots(self, pairs, tensors) -> None:
+        """``dst[a] = src[b]`` (``src`` None: zeros) for every ``(a, b)`` of ``pairs`` and every ``(dst, src)`` of
+        ``tensors``, contiguous with a row of the same size in both, in one launch."""
+        n, T = len(pairs), len(tensors)
+        rows = [dst[0].numel() * dst.element_size() for dst, _ in tensors]
+        rc = self.lib.pih_copy_slots((c_void_p * T)(*(dst.data_ptr() for dst, _ in tensors)),
+                                     (c_void_p * T)(*(0 if src is None else src.data_ptr() for _, src in tensors)),
+                                     (c_ll * T)(*rows), T, (c_int * n)(*(a for a, _ in pairs)),
+                                     (c_int * n)(*(b for _, b in pairs)), n, self._stream())
+        self._check(rc, "copy_slots")
+
     def embedding(self, table: torch.Tensor, ids: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
                   scale: float = 1.0) -> torch.Tensor:
         """``table[ids] * scale``; a scale other than 1 gives 32-bit rows (the product is not rounded again)."""

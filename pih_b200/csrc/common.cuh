@@ -103,6 +103,12 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
+__device__ __forceinline__ float warp_min(float v) {
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, d));
+  return v;
+}
+
 // Sum over a block of up to 1024 threads; every thread gets the result.  The
 // order of additions depends only on blockDim, never on other rows or blocks.
 __device__ __forceinline__ float block_sum(float v, float* scratch /* >= 33 floats */) {

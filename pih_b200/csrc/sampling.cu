@@ -91,7 +91,24 @@ __device__ __forceinline__ uint32_t load_u32_from_block(const uint32_t* local, u
   return v;
 }
 
+// The prefixes are looked for among buckets of scaled values first: kBuckets equal steps from the row's maximum down to
+// its minimum, or 31 below the maximum if that is nearer (a mass is zero from 30.5 on), with the count and the mass of
+// each.  Every wanted prefix ends inside one bucket, whose elements — a few hundred of 150 000 — are collected and ranked
+// one by one.  So a row takes two passes with arithmetic (maximum, buckets) and one of comparisons for each prefix, where
+// radix passes alone (find_crossing: four for each prefix with an exponential an element, then the ties) took 147 us for
+// 32 rows of 151 936, this 55 to 65 us (one row: 27 us, and 5 to 10 us more for each of top_k and top_p); they remain for rows whose crossing falls into a bucket of more than kListed elements (many equal logits, a
+// top_k beyond 31), and for rows with a value that is not finite.
+constexpr int kBuckets = 1984, kOwned = kBuckets / kSampleCluster, kBucketRange = 31;
+constexpr int kListed = 1024, kListedHere = 512;
+
 struct SampleShared {
+  union {
+    uint32_t wide[4][kBuckets];                          // this block's counts and masses in three limbs, a bucket
+    struct {
+      unsigned long long order[kListed], mass[kListed];  // the elements of a bucket: (~key, id), ascending is sorted order
+      unsigned long long here[kListedHere];              // this block's
+    } list;
+    struct {
   // this block's counts of a radix pass, two in turn, as three limbs of 15 bits each summed in 32 bits (a block's
   // part is at most 2^16 ids): 32-bit additions to shared memory are one instruction, 64-bit ones a loop
   uint32_t hist[2][3][256];
@@ -100,13 +117,19 @@ struct SampleShared {
   // adding up a warp's lanes per digit first — match.any, redux.sync — no better, because a warp's dozen distinct
   // digits are worked off one after the other as well).
   uint32_t priv[kSampleCopies][3][256];
+    };
+  };
+  uint32_t owned_count[kOwned];                          // buckets rank * kOwned ...: the row's
+  unsigned long long rank_count[kSampleCluster], rank_mass[kSampleCluster];   // and the sums of every rank's
+  int listed;
+  unsigned long long won[3];                             // the element that was found, count and mass up to it
   unsigned long long ghist[256];                         // the row's
   unsigned long long mine[2][kExchangeWords];            // this block's words of an exchange, two in turn
   unsigned long long all[kSampleCluster][kExchangeWords];
   unsigned long long scratch[40];
   int iscratch[40];
   int sup[kMaxSuppressed];
-  float val[32];
+  float val[32], low[32];
   int idx[32];
   uint32_t prefix_val;
   unsigned long long acc;
@@ -206,6 +229,12 @@ __device__ unsigned long long prefix_total(SampleShared& sm, RowView& rv, const 
 // the first radix pass yields on the way (a pass over the row saved): the least total that is at least `share` of
 // it (kTargetShare: top_p) or the place of the draw `share` in it (kTargetDraw).
 enum TargetKind { kTargetGiven, kTargetShare, kTargetDraw };
+__device__ __forceinline__ unsigned long long target_in(TargetKind kind, double share, unsigned long long total) {
+  const unsigned long long target = kind == kTargetShare ? __double2ull_ru(share * static_cast<double>(total))
+                                                         : __double2ull_rd(share * static_cast<double>(total)) + 1ull;
+  return min(max(target, 1ull), total);
+}
+
 __device__ Prefix find_crossing(SampleShared& sm, RowView& rv, const Prefix& p, bool use_mass, TargetKind kind,
                                 unsigned long long target, double share) {
   if (threadIdx.x == 0) {
@@ -262,9 +291,7 @@ __device__ Prefix find_crossing(SampleShared& sm, RowView& rv, const Prefix& p, 
       // the total of p: the sum of the first pass's counts (every block has the same counts and finds the same)
       unsigned long long total = 0;
       for (int i = 0; i < 256; ++i) total += sm.ghist[i];
-      if (kind == kTargetShare) target = __double2ull_ru(share * static_cast<double>(total));
-      else target = __double2ull_rd(share * static_cast<double>(total)) + 1ull;
-      target = min(max(target, 1ull), total);
+      target = target_in(kind, share, total);
     }
     // the digit at which the running total, from the largest digit down, reaches the target: warp 0, a lane per
     // eight digits (lane 0 the largest), a scan over the lanes' sums, then the lane that holds the crossing walks
@@ -411,6 +438,204 @@ __device__ Prefix find_crossing(SampleShared& sm, RowView& rv, const Prefix& p, 
   return out;
 }
 
+// This rank's running totals from the largest bucket down: warp 0 finds the first of its buckets where the running total
+// (count or mass) reaches target, starting from `count` and `mass`, and leaves (bucket, count, mass in front of it) in won.
+__device__ void find_owned(SampleShared& sm, uint32_t rank, bool use_mass, unsigned long long target, unsigned long long count,
+                           unsigned long long mass) {
+  const int ln = threadIdx.x;
+  unsigned long long c[8], m[8], cs = 0, ms = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int b = ln * 8 + j;
+    c[j] = b < kOwned ? sm.owned_count[b] : 0ull;
+    m[j] = b < kOwned ? sm.ghist[b] : 0ull;
+    cs += c[j];
+    ms += m[j];
+  }
+  unsigned long long ci = cs, mi = ms;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const unsigned long long cn = __shfl_up_sync(0xffffffffu, ci, d), mn = __shfl_up_sync(0xffffffffu, mi, d);
+    if (ln >= d) {
+      ci += cn;
+      mi += mn;
+    }
+  }
+  count += ci - cs;
+  mass += mi - ms;
+  const unsigned long long at = use_mass ? mass : count, all = use_mass ? ms : cs;
+  if (at < target && at + all >= target) {                 // one lane's
+    int b = ln * 8;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if ((use_mass ? mass + m[j] : count + c[j]) >= target) break;
+      mass += m[j];
+      count += c[j];
+      ++b;
+    }
+    sm.won[0] = static_cast<unsigned long long>(rank * kOwned + b);
+    sm.won[1] = count;
+    sm.won[2] = mass;
+  }
+}
+
+// Where the search stands: the bucket whose elements are listed (-1: none), the count and mass in front of it, the
+// elements, and the mass up to the last prefix that was found.
+struct Buckets {
+  float per_unit;
+  int listed_bucket, elements;
+  unsigned long long count_before, mass_before, mass_upto;
+};
+
+__device__ __forceinline__ int bucket_of(const RowView& rv, const Buckets& bk, float scaled) {
+  return min(kBuckets - 1, static_cast<int>((rv.max_scaled - scaled) * bk.per_unit));
+}
+
+// The counts and masses of all buckets.
+__device__ void fill_buckets(SampleShared& sm, RowView& rv, Buckets& bk) {
+  for (int i = threadIdx.x; i < 4 * kBuckets; i += blockDim.x) (&sm.wide[0][0])[i] = 0;
+  __syncthreads();
+  for (int id = rv.lo + threadIdx.x; id < rv.hi; id += blockDim.x) {
+    if (!allowed(rv, id)) continue;
+    const float s = rv.staged[id - rv.lo];
+    const int b = bucket_of(rv, bk, s);
+    const unsigned long long a = mass_of(rv, s);
+    const uint32_t a0 = static_cast<uint32_t>(a) & 0x7FFFu, a1 = static_cast<uint32_t>(a >> 15) & 0x7FFFu,
+                   a2 = static_cast<uint32_t>(a >> 30);
+    atomicAdd(&sm.wide[0][b], 1u);
+    if (a0) atomicAdd(&sm.wide[1][b], a0);
+    if (a1) atomicAdd(&sm.wide[2][b], a1);
+    if (a2) atomicAdd(&sm.wide[3][b], a2);
+  }
+  sample_cluster_sync();
+  unsigned long long count = 0, mass = 0;
+  if (threadIdx.x < kOwned) {
+    uint32_t part[kSampleCluster][4];
+#pragma unroll
+    for (int r = 0; r < kSampleCluster; ++r)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) part[r][k] = load_u32_from_block(&sm.wide[k][rv.rank * kOwned + threadIdx.x], r);
+#pragma unroll
+    for (int r = 0; r < kSampleCluster; ++r) {
+      count += part[r][0];
+      mass += static_cast<unsigned long long>(part[r][1]) + (static_cast<unsigned long long>(part[r][2]) << 15) +
+              (static_cast<unsigned long long>(part[r][3]) << 30);
+    }
+    sm.owned_count[threadIdx.x] = static_cast<uint32_t>(count);
+    sm.ghist[threadIdx.x] = mass;
+  }
+  const unsigned long long w[kExchangeWords] = {block_sum_u64(count, sm.scratch), block_sum_u64(mass, sm.scratch), 0ull, 0ull};
+  exchange(sm, rv, w);
+  if (threadIdx.x < kSampleCluster) {
+    sm.rank_count[threadIdx.x] = sm.all[threadIdx.x][0];
+    sm.rank_mass[threadIdx.x] = sm.all[threadIdx.x][1];
+  }
+  __syncthreads();
+  bk.mass_upto = 0;
+  for (int r = 0; r < kSampleCluster; ++r) bk.mass_upto += sm.rank_mass[r];
+}
+
+// The first place where the running total reaches target (count or mass; at most the total up to the last prefix found);
+// false: its bucket holds too many elements.  All blocks of the cluster find the same.
+__device__ bool find_in_buckets(SampleShared& sm, RowView& rv, Buckets& bk, bool use_mass, unsigned long long target, Prefix* out) {
+  if (bk.listed_bucket < 0 || !use_mass || target <= bk.mass_before) {
+    unsigned long long count = 0, mass = 0;
+    int owner = -1;
+    for (int r = 0; r < kSampleCluster; ++r) {
+      const unsigned long long c = sm.rank_count[r], m = sm.rank_mass[r];
+      if ((use_mass ? mass + m : count + c) >= target) {
+        owner = r;
+        break;
+      }
+      count += c;
+      mass += m;
+    }
+    if (owner < 0) return false;
+    if (rv.rank == static_cast<uint32_t>(owner) && threadIdx.x < 32) find_owned(sm, rv.rank, use_mass, target, count, mass);
+    if (threadIdx.x == 0) sm.listed = 0;
+    __syncthreads();
+    {
+      const unsigned long long w[kExchangeWords] = {sm.won[0], sm.won[1], sm.won[2], 0ull};
+      exchange(sm, rv, w);
+    }
+    const int b = static_cast<int>(sm.all[owner][0]);
+    bk.count_before = sm.all[owner][1];
+    bk.mass_before = sm.all[owner][2];
+    bk.listed_bucket = b;
+    for (int id = rv.lo + threadIdx.x; id < rv.hi; id += blockDim.x) {
+      const float s = rv.staged[id - rv.lo];
+      if (bucket_of(rv, bk, s) != b || !allowed(rv, id)) continue;
+      const int at = atomicAdd(&sm.listed, 1);
+      if (at < kListedHere)
+        sm.list.here[at] = (static_cast<unsigned long long>(~ordered_key(s)) << 32) | static_cast<uint32_t>(id);
+    }
+    __syncthreads();
+    {
+      const unsigned long long w[kExchangeWords] = {static_cast<unsigned long long>(sm.listed), 0ull, 0ull, 0ull};
+      exchange(sm, rv, w);
+    }
+    int n = 0;
+    bool fits = true;
+    for (int r = 0; r < kSampleCluster; ++r) {
+      fits = fits && sm.all[r][0] <= static_cast<unsigned long long>(kListedHere);
+      n += static_cast<int>(sm.all[r][0]);
+    }
+    if (!fits || n > kListed) return false;                // (before anything is written where the radix passes count)
+    for (int r = 0, at = 0; r < kSampleCluster; at += static_cast<int>(sm.all[r][0]), ++r) {
+      for (int i = threadIdx.x; i < static_cast<int>(sm.all[r][0]); i += blockDim.x) {
+        const unsigned long long o = load_u64_from_block(&sm.list.here[i], r);
+        const uint32_t key = ~static_cast<uint32_t>(o >> 32);
+        const float s = __uint_as_float((key & 0x80000000u) ? key ^ 0x80000000u : ~key);
+        sm.list.order[at + i] = o;
+        sm.list.mass[at + i] = mass_of(rv, s);
+      }
+    }
+    bk.elements = n;
+  }
+  __syncthreads();
+  // a warp an element, the elements shared out among the blocks: the count and mass up to and with it
+  const unsigned long long want = target - (use_mass ? bk.mass_before : bk.count_before);
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  if (threadIdx.x == 0) sm.won[1] = 0ull;
+  __syncthreads();
+  for (int i = static_cast<int>(rv.rank) + kSampleCluster * (threadIdx.x >> 5); i < bk.elements; i += kSampleCluster * warps) {
+    const unsigned long long mine = sm.list.order[i], weight = use_mass ? sm.list.mass[i] : 1ull;
+    int count = 0;
+    unsigned long long mass = 0;
+    for (int j = lane; j < bk.elements; j += 32) {
+      if (sm.list.order[j] <= mine) {
+        ++count;
+        mass += sm.list.mass[j];
+      }
+    }
+    count = __reduce_add_sync(0xffffffffu, count);
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) mass += __shfl_xor_sync(0xffffffffu, mass, d);
+    const unsigned long long upto = use_mass ? mass : static_cast<unsigned long long>(count);
+    if (lane == 0 && upto >= want && upto - weight < want) {   // one element's (a weight of zero reaches nothing)
+      sm.won[0] = mine;
+      sm.won[1] = 1ull;
+      sm.won[2] = mass;
+    }
+  }
+  __syncthreads();
+  {
+    const unsigned long long w[kExchangeWords] = {sm.won[0], sm.won[1], sm.won[2], 0ull};
+    exchange(sm, rv, w);
+  }
+  unsigned long long order = 0, mass = 0;
+  for (int r = 0; r < kSampleCluster; ++r)
+    if (sm.all[r][1] != 0ull) {
+      order = sm.all[r][0];
+      mass = sm.all[r][2];
+    }
+  out->key = ~static_cast<uint32_t>(order >> 32);
+  out->id = static_cast<int>(static_cast<uint32_t>(order));
+  bk.mass_upto = bk.mass_before + mass;
+  __syncthreads();
+  return true;
+}
+
 __global__ void __launch_bounds__(kSampleBlock)
 sample_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ fparams,
               const int* __restrict__ iparams, int* __restrict__ out_tokens, int staged_floats, uint32_t* error) {
@@ -447,18 +672,30 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
   extern __shared__ float staged_part[];
   bool bad = false;
   // maximum and its lowest id, found on the way
-  float best = -INFINITY;
+  float best = -INFINITY, least = INFINITY;
   int best_id = 0x7fffffff;
   const bool stage = staged_floats >= rv.hi - rv.lo;
-  for (int id = rv.lo + threadIdx.x; id < rv.hi; id += blockDim.x) {
-    const float raw = rv.logits[id];
-    if (!isfinite(raw)) bad = true;
-    const float s = raw / rv.temperature;
-    if (stage) staged_part[id - rv.lo] = s;
-    if (!allowed(rv, id)) continue;
-    if (s > best || (s == best && id < best_id)) {
-      best = s;
-      best_id = id;
+  constexpr int kAhead = 8;                              // loads asked for together
+  for (int first = rv.lo + threadIdx.x; first < rv.hi; first += kAhead * blockDim.x) {
+    float ahead[kAhead];
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) {
+      const int id = first + i * blockDim.x;
+      ahead[i] = id < rv.hi ? rv.logits[id] : 0.0f;
+    }
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) {
+      const int id = first + i * blockDim.x;
+      if (id >= rv.hi) break;
+      if (!isfinite(ahead[i])) bad = true;
+      const float s = ahead[i] / rv.temperature;
+      if (stage) staged_part[id - rv.lo] = s;
+      if (!allowed(rv, id)) continue;
+      least = fminf(least, s);
+      if (s > best || (s == best && id < best_id)) {
+        best = s;
+        best_id = id;
+      }
     }
   }
   if (stage) rv.staged = staged_part;                    // (read only after the block barriers of the reduction below)
@@ -468,6 +705,7 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
   for (int d = 16; d > 0; d >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, best, d);
     const int oi = __shfl_xor_sync(0xffffffffu, best_id, d);
+    least = fminf(least, __shfl_xor_sync(0xffffffffu, least, d));
     if (ov > best || (ov == best && oi < best_id)) {
       best = ov;
       best_id = oi;
@@ -476,9 +714,11 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
   if (lane == 0) {
     sm.val[warp] = best;
     sm.idx[warp] = best_id;
+    sm.low[warp] = least;
   }
-  __syncthreads();
+  const bool any_bad = __syncthreads_or(bad);
   if (warp == 0) {
+    least = warp_min(lane < (blockDim.x >> 5) ? sm.low[lane] : INFINITY);
     best = lane < (blockDim.x >> 5) ? sm.val[lane] : -INFINITY;
     best_id = lane < (blockDim.x >> 5) ? sm.idx[lane] : 0x7fffffff;
 #pragma unroll
@@ -493,20 +733,26 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
     if (lane == 0) {
       sm.val[0] = best;
       sm.idx[0] = best_id;
+      sm.low[0] = least;
     }
   }
   __syncthreads();
   {
     const unsigned long long w[kExchangeWords] = {static_cast<unsigned long long>(__float_as_uint(sm.val[0])),
-                                                  static_cast<unsigned long long>(static_cast<uint32_t>(sm.idx[0])), 0ull, 0ull};
+                                                  static_cast<unsigned long long>(static_cast<uint32_t>(sm.idx[0])),
+                                                  static_cast<unsigned long long>(__float_as_uint(sm.low[0])), any_bad || !stage ? 1ull : 0ull};
     exchange(sm, rv, w);
   }
+  bool by_buckets = true;
+  least = INFINITY;
   best = -INFINITY;
   best_id = 0x7fffffff;
 #pragma unroll
   for (int r = 0; r < kSampleCluster; ++r) {             // the blocks' ids ascend with their rank: the first maximum has the lowest id
     const float v = __uint_as_float(static_cast<uint32_t>(sm.all[r][0]));
     const int i = static_cast<int>(static_cast<uint32_t>(sm.all[r][1]));
+    least = fminf(least, __uint_as_float(static_cast<uint32_t>(sm.all[r][2])));
+    by_buckets = by_buckets && sm.all[r][3] == 0ull;
     if (v > best || (v == best && i < best_id)) {
       best = v;
       best_id = i;
@@ -525,16 +771,26 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
   kept.key = 0u;
   kept.id = 0x7fffffff;
   const int n_allowed = vocab - nsup;
-  if (top_k > 0 && top_k < n_allowed)
-    kept = find_crossing(sm, rv, kept, false, kTargetGiven, static_cast<unsigned long long>(top_k), 0.0);
-  if (top_p < 1.0f) {
-    kept = find_crossing(sm, rv, kept, true, kTargetShare, 0ull, static_cast<double>(top_p));
-  }
   const uint32_t word = philox_word(static_cast<uint32_t>(ip[1]), static_cast<uint32_t>(ip[2]),
                                     (static_cast<uint64_t>(static_cast<uint32_t>(ip[4])) << 32) |
                                         static_cast<uint32_t>(ip[3]));
   const double u = (static_cast<double>(word) + 0.5) / 4294967296.0;
-  const Prefix pick = find_crossing(sm, rv, kept, true, kTargetDraw, 0ull, u);
+  Buckets bk = {0.0f, -1, 0, 0ull, 0ull, 0ull};
+  if (by_buckets) {
+    bk.per_unit = static_cast<float>(kBuckets - 1) / fmaxf(fminf(best - least, static_cast<float>(kBucketRange)), 1e-6f);
+    fill_buckets(sm, rv, bk);
+  }
+  if (top_k > 0 && top_k < n_allowed) {
+    by_buckets = by_buckets && find_in_buckets(sm, rv, bk, false, static_cast<unsigned long long>(top_k), &kept);
+    if (!by_buckets) kept = find_crossing(sm, rv, kept, false, kTargetGiven, static_cast<unsigned long long>(top_k), 0.0);
+  }
+  if (top_p < 1.0f) {
+    by_buckets = by_buckets && find_in_buckets(sm, rv, bk, true, target_in(kTargetShare, static_cast<double>(top_p), bk.mass_upto), &kept);
+    if (!by_buckets) kept = find_crossing(sm, rv, kept, true, kTargetShare, 0ull, static_cast<double>(top_p));
+  }
+  Prefix pick = kept;
+  by_buckets = by_buckets && find_in_buckets(sm, rv, bk, true, target_in(kTargetDraw, u, bk.mass_upto), &pick);
+  if (!by_buckets) pick = find_crossing(sm, rv, kept, true, kTargetDraw, 0ull, u);
   if (threadIdx.x == 0 && rv.rank == 0) out_tokens[row] = pick.id;
   sample_cluster_sync();                                 // nobody leaves while another block may still read its words
 }
@@ -1007,7 +1263,7 @@ extern "C" int pih_sample(const float* logits, int rows, int vocab, const float*
   }
   if (static_cast<long long>(part) * 4 > room) staged_floats = 0;
   static int smem_set = 0;
-  if (staged_floats * 4 > 40 * 1024 && smem_set < staged_floats * 4) {
+  if (staged_floats * 4 > smem_set) {
     cudaError_t e = cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, staged_floats * 4);
     if (e != cudaSuccess) return static_cast<int>(e);
     smem_set = staged_floats * 4;

@@ -7,6 +7,15 @@
 //
 // The order of the additions of a read-out is fixed by the kernel: it does not depend on how a sequence is cut into
 // steps or on what else a step holds.
+//
+// bf16, a step with a request of more than 64 rows: requests of more than 16 rows go by chunks of 64 rows instead, all
+// chunks side by side, in 32-bit products on the CUDA cores (the same precision; the token loop is a chain of 0.27 us a
+// token on 32 of the 148 SMs, 560 us for 2048 rows of 8 heads of 128 x 128):
+//   retention_chunk_state   U = sum_j decay^(end - j) k_j v_j^T, what a chunk adds to the state
+//   retention_state_pass    the chunks in order: the state in front of each takes U's place; S <- decay^rows S + U
+//   retention_chunk_out     o_i = decay^(i + 1) S^T q_i + sum_{j <= i} decay^(i - j) (q_i . k_j) v_j
+// decay^n is formed as exp(n log1p(decay - 1)).
+#include "chunks.cuh"
 #include "common.cuh"
 
 namespace pih {
@@ -58,7 +67,7 @@ __global__ void retention_recurrence_kernel(const float* __restrict__ qf, const 
                                             const T* __restrict__ v, long long ldv, const float* __restrict__ decay_m1,
                                             float* __restrict__ out, float* __restrict__ state, long long state_stride,
                                             const int* __restrict__ cu_q, const int* __restrict__ state_slots, int heads,
-                                            int dim, int vdim) {
+                                            int dim, int vdim, int small_rows) {
   extern __shared__ float smem[];
   wait_for_prior_kernels();
   launch_dependents();
@@ -67,7 +76,7 @@ __global__ void retention_recurrence_kernel(const float* __restrict__ qf, const 
   const int j = threadIdx.x, col = blockIdx.z * cols + j;
   const int lo = cu_q[r], hi = cu_q[r + 1];
   const int slot = state_slots[r];
-  if (hi <= lo || slot < 0) return;
+  if (hi <= lo || slot < 0 || hi - lo > small_rows) return;
   float* S = smem;                          // [dim][cols]
   float* kq = smem + dim * cols;            // [2 buffers][k: dim | q: dim]
   const bool live = col < vdim;
@@ -135,7 +144,7 @@ __global__ void __launch_bounds__(kDim >= 64 ? 256 : (kDim >= 32 ? 128 : 64))
 retention_recurrence_reg_kernel(const float* __restrict__ qf, const float* __restrict__ kf, const T* __restrict__ v,
                                 long long ldv, const float* __restrict__ decay_m1, float* __restrict__ out,
                                 float* __restrict__ state, long long state_stride, const int* __restrict__ cu_q,
-                                const int* __restrict__ state_slots, int heads, int vdim) {
+                                const int* __restrict__ state_slots, int heads, int vdim, int small_rows) {
   constexpr int kParts = kDim >= 64 ? 8 : (kDim >= 32 ? 4 : 2);   // threads a column of S
   constexpr int kThreads = 32 * kParts;
   constexpr int kRows = kDim / kParts;                    // rows of S a thread holds (a multiple of 4)
@@ -151,7 +160,7 @@ retention_recurrence_reg_kernel(const float* __restrict__ qf, const float* __res
   const int r = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * 32;
   const int lo = cu_q[r], hi = cu_q[r + 1];
   const int slot = state_slots[r];
-  if (hi <= lo || slot < 0) return;
+  if (hi <= lo || slot < 0 || hi - lo > small_rows) return;
   const int tid = threadIdx.x, c = tid / kParts, p = tid % kParts;
   float* Sg = state + slot * state_stride + (static_cast<long long>(h) * kDim + p * kRows) * vdim + col0 + c;
   float S[kRows];
@@ -217,15 +226,217 @@ retention_recurrence_reg_kernel(const float* __restrict__ qf, const float* __res
   for (int i = 0; i < kRows; ++i) Sg[static_cast<long long>(i) * vdim] = S[i];
 }
 
+// ---- by chunks ----------------------------------------------------------------------------------------------------------
+constexpr int kRetentionSmallRows = 16;                    // requests of at most this many rows go token by token
+
+struct RetentionArgs {
+  const float* q;                                          // rotated, [rows, heads, dim]
+  const float* k;                                          // rotated and scaled
+  const __nv_bfloat16* v;
+  long long ldv;
+  const float* decay_m1;
+  float* out;
+  float* state;
+  long long state_stride;
+  float* chunk_states;                                     // [chunks, heads, dim, vdim]
+  const int* cu_q;
+  const int* state_slots;
+  int requests, heads, vdim;
+};
+
+__device__ __forceinline__ float decay_power(float log_decay, int n) { return n == 0 ? 1.0f : expf(log_decay * static_cast<float>(n)); }
+
+// Block (chunk, head, VT value columns), 256 threads: DIM / 16 rows by VT / 16 columns of U a thread.  Bound by the FMA
+// units (64 k-steps of 2048 two-number FMAs from 16 KB of shared memory reads).
+template <int DIM, int VT>
+__global__ void __launch_bounds__(256)
+retention_chunk_state_kernel(const RetentionArgs p) {
+  extern __shared__ __align__(16) float smem[];
+  float* ks = smem;                                        // [64][DIM]
+  float* vs = ks + chunks::kRows * DIM;                    // [64][VT]
+  __shared__ chunks::Place place;
+  __shared__ float power[chunks::kRows];
+  wait_for_prior_kernels();
+  launch_dependents();
+  const chunks::Place c = chunks::find(p.cu_q, p.state_slots, p.requests, kRetentionSmallRows, blockIdx.x, &place);
+  if (c.request < 0) return;
+  const int h = blockIdx.y, v0 = blockIdx.z * VT, tid = threadIdx.x;
+  chunks::load_rows<DIM, DIM>(ks, p.k + (static_cast<long long>(c.first) * p.heads + h) * DIM, static_cast<long long>(p.heads) * DIM, c.rows);
+  chunks::copies_commit();
+  if (tid < chunks::kRows) power[tid] = decay_power(log1pf(p.decay_m1[h]), max(0, c.rows - 1 - tid));
+  chunks::load_rows<VT, VT>(vs, p.v + c.first * p.ldv + static_cast<long long>(h) * p.vdim + v0, p.ldv, c.rows);
+  __syncthreads();
+  for (int e = tid; e < chunks::kRows * VT; e += 256) vs[e] *= power[e / VT];
+  chunks::copies_wait();
+  __syncthreads();
+  constexpr int RM = DIM / 16, RN = VT / 16;
+  float2 U[RM][RN / 2];
+  chunks::clear(U);
+  chunks::multiply_outer<RM, RN>(U, ks, DIM, vs, VT, (c.rows + 3) & ~3);
+  const int tx = tid & 15, ty = tid >> 4;
+  float* to = p.chunk_states + ((static_cast<long long>(c.index) * p.heads + h) * DIM + ty * RM) * p.vdim + v0 + 4 * tx;
+#pragma unroll
+  for (int i = 0; i < RM; ++i)
+#pragma unroll
+    for (int g = 0; g < RN / 4; ++g)
+      *reinterpret_cast<float4*>(to + static_cast<long long>(i) * p.vdim + 64 * g) =
+          make_float4(U[i][2 * g].x, U[i][2 * g].y, U[i][2 * g + 1].x, U[i][2 * g + 1].y);
+}
+
+// Block (request, head, 128 pieces of four numbers of S): a stream over the chunks, eight of them asked for ahead.
+__global__ void __launch_bounds__(128)
+retention_state_pass_kernel(const RetentionArgs p, int dim) {
+  __shared__ int first;
+  wait_for_prior_kernels();
+  launch_dependents();
+  const int r = blockIdx.x, h = blockIdx.y;
+  const int n = p.cu_q[r + 1] - p.cu_q[r], slot = p.state_slots[r];
+  if (n <= kRetentionSmallRows || slot < 0) return;
+  if (threadIdx.x == 0) first = chunks::first_of(p.cu_q, p.state_slots, kRetentionSmallRows, r);
+  __syncthreads();
+  const long long matrix = static_cast<long long>(dim) * p.vdim, at = (static_cast<long long>(blockIdx.z) * 128 + threadIdx.x) * 4;
+  if (at >= matrix) return;
+  float* Sg = p.state + slot * p.state_stride + h * matrix + at;
+  float4 S = make_float4(Sg[0], Sg[1], Sg[2], Sg[3]);
+  float* U = p.chunk_states + (static_cast<long long>(first) * p.heads + h) * matrix + at;
+  const long long step = p.heads * matrix;
+  const int count = (n + chunks::kRows - 1) / chunks::kRows;
+  const float lg = log1pf(p.decay_m1[h]), whole = decay_power(lg, chunks::kRows);
+  constexpr int kAhead = 8;
+  float4 u[kAhead];
+#pragma unroll
+  for (int i = 0; i < kAhead; ++i)
+    if (i < count) u[i] = *reinterpret_cast<const float4*>(U + i * step);
+  for (int c0 = 0; c0 < count; c0 += kAhead) {
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) {
+      const int c = c0 + i;
+      if (c >= count) break;
+      const float4 add = u[i];
+      if (c + kAhead < count) u[i] = *reinterpret_cast<const float4*>(U + (c + kAhead) * step);
+      *reinterpret_cast<float4*>(U + c * step) = S;
+      const float f = c + 1 < count ? whole : decay_power(lg, n - c * chunks::kRows);
+      S.x = fmaf(f, S.x, add.x);
+      S.y = fmaf(f, S.y, add.y);
+      S.z = fmaf(f, S.z, add.z);
+      S.w = fmaf(f, S.w, add.w);
+    }
+  }
+  Sg[0] = S.x; Sg[1] = S.y; Sg[2] = S.z; Sg[3] = S.w;
+}
+
+template <int DIM, int VT>
+constexpr size_t retention_out_bytes() {
+  return sizeof(float) * chunks::kRows * (2 * (DIM + 4) + (VT > DIM + 4 ? VT - DIM - 4 : 0) + 68);
+}
+
+// Block (chunk, head, VT value columns), 256 threads: 4 rows by VT / 16 columns of the read-outs a thread.
+template <int DIM, int VT>
+__global__ void __launch_bounds__(256, 2)
+retention_chunk_out_kernel(const RetentionArgs p) {
+  constexpr int LD = DIM + 4, LP = 68;
+  extern __shared__ __align__(16) float smem[];
+  float* qs = smem;                                        // [64][LD]
+  float* P = qs + chunks::kRows * LD;                      // [64][LP]: decayed scores
+  float* ks = P + chunks::kRows * LP;                      // [64][LD]; then 64 rows of the state [64][VT]; then the values
+  __shared__ chunks::Place place;
+  __shared__ float power[chunks::kRows + 1];
+  wait_for_prior_kernels();
+  launch_dependents();
+  const chunks::Place c = chunks::find(p.cu_q, p.state_slots, p.requests, kRetentionSmallRows, blockIdx.x, &place);
+  if (c.request < 0) return;
+  const int h = blockIdx.y, v0 = blockIdx.z * VT, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const long long at = (static_cast<long long>(c.first) * p.heads + h) * DIM, ld = static_cast<long long>(p.heads) * DIM;
+  chunks::load_rows<DIM, LD>(qs, p.q + at, ld, c.rows);
+  chunks::load_rows<DIM, LD>(ks, p.k + at, ld, c.rows);
+  chunks::copies_commit();
+  if (tid <= chunks::kRows) power[tid] = decay_power(log1pf(p.decay_m1[h]), tid);
+  chunks::copies_wait();
+  __syncthreads();
+  {
+    float2 s[4][4];
+    chunks::clear(s);
+    chunks::multiply_rows<4, 4, DIM, LD>(s, qs, ks);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int row = ty * 4 + i, col = tx + 16 * j;
+        P[row * LP + col] = col <= row ? (s[i][j].x + s[i][j].y) * power[row - col] : 0.0f;
+      }
+  }
+  constexpr int RN = VT / 16;
+  float2 o[4][RN / 2];
+  chunks::clear(o);
+  const float* state = p.chunk_states + (static_cast<long long>(c.index) * p.heads + h) * DIM * p.vdim + v0;
+#pragma unroll 1
+  for (int d0 = 0; d0 < DIM; d0 += chunks::kRows) {
+    __syncthreads();                                       // (what lay there is done with)
+    chunks::load_rows<VT, VT>(ks, state + static_cast<long long>(d0) * p.vdim, p.vdim, chunks::kRows);
+    chunks::copies_commit();
+    chunks::copies_wait();
+    __syncthreads();
+    chunks::multiply_columns<4, RN>(o, qs + d0, LD, ks, VT, chunks::kRows);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < RN / 2; ++j) {
+      o[i][j].x *= power[ty * 4 + i + 1];
+      o[i][j].y *= power[ty * 4 + i + 1];
+    }
+  __syncthreads();
+  chunks::load_rows<VT, VT>(ks, p.v + c.first * p.ldv + static_cast<long long>(h) * p.vdim + v0, p.ldv, c.rows);
+  __syncthreads();
+  chunks::multiply_columns<4, RN>(o, P, LP, ks, VT, (tid >> 5) * 8 + 8);       // (the warp's rows see no later ones)
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int row = ty * 4 + i;
+    if (row >= c.rows) continue;
+    float* to = p.out + (static_cast<long long>(c.first + row) * p.heads + h) * p.vdim + v0 + 4 * tx;
+#pragma unroll
+    for (int g = 0; g < RN / 4; ++g)
+      *reinterpret_cast<float4*>(to + 64 * g) = make_float4(o[i][2 * g].x, o[i][2 * g].y, o[i][2 * g + 1].x, o[i][2 * g + 1].y);
+  }
+}
+
 }  // namespace pih
 
 using namespace pih;
 typedef __nv_bfloat16 bf16;
 
+// Steps that may go by chunks: bf16 values that can be read 16 bytes at a time, sizes with an instance.
+static bool retention_takes_chunks(int dtype, const void* v, long long ldv, int heads, int dim, int vdim) {
+  return dtype == PIH_BF16 && (dim == 64 || dim == 128) && vdim % 64 == 0 && heads <= 65535 && vdim / 64 <= 65535 &&
+         reinterpret_cast<uintptr_t>(v) % 16 == 0 && ldv % 8 == 0;
+}
+
+// fp32 numbers of chunk scratch that a step of ``rows`` rows needs; 0: its sizes do not go by chunks.
+extern "C" long long pih_retention_chunk_scratch(int dtype, const void* v, long long ldv, int rows, int requests, int heads, int dim,
+                                                 int vdim) {
+  if (!retention_takes_chunks(dtype, v, ldv, heads, dim, vdim)) return 0;
+  return chunks::at_most(rows, requests, kRetentionSmallRows) * heads * dim * vdim;
+}
+
+template <int DIM, int VT>
+static int launch_retention_chunks(cudaStream_t s, const RetentionArgs& p, int rows) {
+  const unsigned count = static_cast<unsigned>(chunks::at_most(rows, p.requests, kRetentionSmallRows)), tiles = p.vdim / VT;
+  constexpr size_t state_bytes = sizeof(float) * chunks::kRows * (DIM + VT), out_bytes = retention_out_bytes<DIM, VT>();
+  cudaFuncSetAttribute(retention_chunk_state_kernel<DIM, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(state_bytes));
+  cudaFuncSetAttribute(retention_chunk_out_kernel<DIM, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(out_bytes));
+  launch_kernel(retention_chunk_state_kernel<DIM, VT>, dim3(count, p.heads, tiles), dim3(256), state_bytes, s, p);
+  PIH_LAUNCH_CHECK();
+  launch_kernel(retention_state_pass_kernel, dim3(p.requests, p.heads, (DIM * p.vdim / 4 + 127) / 128), dim3(128), 0, s, p, DIM);
+  PIH_LAUNCH_CHECK();
+  launch_kernel(retention_chunk_out_kernel<DIM, VT>, dim3(count, p.heads, tiles), dim3(256), out_bytes, s, p);
+  PIH_LAUNCH_CHECK();
+  return 0;
+}
+
 template <typename T, int D>
 static void launch_retention_in_registers(cudaStream_t s, const float* qf, const float* kf, const void* v, long long ldv,
                                           const void* decay_m1, void* out, void* state, long long state_stride,
-                                          const void* cu_q, const void* state_slots, int requests, int heads, int vdim) {
+                                          const void* cu_q, const void* state_slots, int requests, int heads, int vdim, int small_rows) {
   constexpr int parts = D >= 64 ? 8 : (D >= 32 ? 4 : 2);
   constexpr int chunk = D <= 128 ? 16 : 8;
   constexpr size_t needed = 2 * chunk * (2 * parts * (D / parts + 4) + 32 * sizeof(T) / 4) * sizeof(float);
@@ -239,17 +450,23 @@ static void launch_retention_in_registers(cudaStream_t s, const float* qf, const
   launch_kernel(retention_recurrence_reg_kernel<T, D>, dim3(requests, heads, vdim / 32), dim3(32 * parts), bytes, s, qf, kf,
                 static_cast<const T*>(v), ldv, static_cast<const float*>(decay_m1), static_cast<float*>(out),
                 static_cast<float*>(state), state_stride, static_cast<const int*>(cu_q),
-                static_cast<const int*>(state_slots), heads, vdim);
+                static_cast<const int*>(state_slots), heads, vdim, small_rows);
 }
 
 // qk [rows, ld]: q heads then k heads ([heads, dim] each); v [rows, ldv]: [heads, vdim]; freq fp32 [rot / 2] (null: no
 // rotation); decay_m1 fp32 [heads]: decay - 1; scratch fp32 [2 * rows * heads * dim]; out fp32 [rows, heads, vdim];
-// state fp32: S of (slot, head) at state + slot * state_stride + head * dim * vdim, [dim, vdim].
+// state fp32: S of (slot, head) at state + slot * state_stride + head * dim * vdim, [dim, vdim].  chunk_scratch: null, or
+// pih_retention_chunk_scratch numbers, 16-byte aligned: requests of more than 16 rows go by chunks; ``small`` 0 then says that
+// there are no others.
 extern "C" int pih_retention(int dtype, const void* qk, long long ld, const void* v, long long ldv, const void* freq, int rot,
                              const void* positions, const void* decay_m1, float key_scale, void* scratch, void* out,
                              void* state, long long state_stride, const void* cu_q, const void* state_slots, int rows,
-                             int requests, int heads, int dim, int vdim, void* stream) {
+                             int requests, int heads, int dim, int vdim, void* chunk_scratch, int small, void* stream) {
   if (rows <= 0 || requests <= 0) return 0;
+  if (chunk_scratch != nullptr && (!retention_takes_chunks(dtype, v, ldv, heads, dim, vdim) ||
+                                   reinterpret_cast<uintptr_t>(chunk_scratch) % 16 || reinterpret_cast<uintptr_t>(scratch) % 16))
+    return PIH_ERR_UNSUPPORTED;
+  const int small_rows = chunk_scratch != nullptr ? kRetentionSmallRows : 0x7fffffff;
   if (rot < 0 || rot > dim || (rot & 1) || (rot > 0 && freq == nullptr)) return PIH_ERR_BAD_ARGUMENT;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int cols = vdim >= 64 ? 64 : 32;
@@ -266,13 +483,24 @@ extern "C" int pih_retention(int dtype, const void* qk, long long ld, const void
   const bool in_registers = (dim == 16 || dim == 32 || dim == 64 || dim == 128 || dim == 256) && vdim % 32 == 0 &&
                             (reinterpret_cast<uintptr_t>(v) % 16 == 0) && (ldv * esize) % 16 == 0 &&
                             (vdim * esize) % 16 == 0 && (reinterpret_cast<uintptr_t>(scratch) % 16 == 0);
-#define PIH_RET_ARGS s, qf, kf, v, ldv, decay_m1, out, state, state_stride, cu_q, state_slots, requests, heads, vdim
+#define PIH_RET_ARGS s, qf, kf, v, ldv, decay_m1, out, state, state_stride, cu_q, state_slots, requests, heads, vdim, small_rows
 #define PIH_RET(T)                                                                                                     \
   do {                                                                                                                 \
     launch_kernel(retention_prepare_kernel<T>, dim3(static_cast<unsigned>((n + 255) / 256)), dim3(256), 0, s,          \
                   static_cast<const T*>(qk), ld, static_cast<const float*>(freq), static_cast<const int*>(positions),  \
                   qf, kf, rows, heads, dim, rot, key_scale);                                                           \
     PIH_LAUNCH_CHECK();                                                                                                \
+    if (chunk_scratch != nullptr) {                                                                                    \
+      const RetentionArgs p = {qf, kf, static_cast<const bf16*>(v), ldv, static_cast<const float*>(decay_m1),          \
+                               static_cast<float*>(out), static_cast<float*>(state), state_stride,                     \
+                               static_cast<float*>(chunk_scratch), static_cast<const int*>(cu_q),                      \
+                               static_cast<const int*>(state_slots), requests, heads, vdim};                           \
+      const int rc = dim == 128 ? (vdim % 128 ? launch_retention_chunks<128, 64>(s, p, rows)                           \
+                                              : launch_retention_chunks<128, 128>(s, p, rows))                         \
+                                : (vdim % 128 ? launch_retention_chunks<64, 64>(s, p, rows)                            \
+                                              : launch_retention_chunks<64, 128>(s, p, rows));                         \
+      if (rc != 0 || !small) return rc;                                                                                \
+    }                                                                                                                  \
     if (in_registers) {                                                                                                \
       switch (dim) {                                                                                                   \
         case 16: launch_retention_in_registers<T, 16>(PIH_RET_ARGS); break;                                           \
@@ -289,7 +517,7 @@ extern "C" int pih_retention(int dtype, const void* qk, long long ld, const void
     launch_kernel(retention_recurrence_kernel<T>, grid, dim3(cols), smem, s, static_cast<const float*>(qf),            \
                   static_cast<const float*>(kf), static_cast<const T*>(v), ldv, static_cast<const float*>(decay_m1),   \
                   static_cast<float*>(out), static_cast<float*>(state), state_stride, static_cast<const int*>(cu_q),   \
-                  static_cast<const int*>(state_slots), heads, dim, vdim);                                             \
+                  static_cast<const int*>(state_slots), heads, dim, vdim, small_rows);                                 \
   } while (0)
   if (dtype == PIH_F32) PIH_RET(float);
   else if (dtype == PIH_BF16) PIH_RET(bf16);

@@ -96,8 +96,9 @@ __device__ __forceinline__ uint32_t load_u32_from_block(const uint32_t* local, u
 // each.  Every wanted prefix ends inside one bucket, whose elements — a few hundred of 150 000 — are collected and ranked
 // one by one.  So a row takes two passes with arithmetic (maximum, buckets) and one of comparisons for each prefix, where
 // radix passes alone (find_crossing: four for each prefix with an exponential an element, then the ties) took 147 us for
-// 32 rows of 151 936, this 55 to 65 us (one row: 27 us, and 5 to 10 us more for each of top_k and top_p); they remain for rows whose crossing falls into a bucket of more than kListed elements (many equal logits, a
-// top_k beyond 31), and for rows with a value that is not finite.
+// 32 rows of 151 936, this 55 to 65 us (one row: 27 us, and 5 to 10 us more for each of top_k and top_p).  They remain
+// for rows whose crossing falls into a bucket of more than kListed elements (many equal logits, a top_k beyond 31), and
+// for rows with a value that is not finite.
 constexpr int kBuckets = 1984, kOwned = kBuckets / kSampleCluster, kBucketRange = 31;
 constexpr int kListed = 1024, kListedHere = 512;
 

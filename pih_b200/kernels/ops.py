@@ -119,6 +119,7 @@ class CudaOps:
         lib.pih_top_logprobs_scratch_words.restype = c_ll
         lib.pih_moe_route_words.restype = c_ll
         lib.pih_linear_memory_scratch.restype = c_ll
+        lib.pih_retention_chunk_scratch.restype = c_ll
 
     def _native_supports(self, block) -> bool:
         from .native_block import NativeBlocks
@@ -1159,13 +1160,29 @@ class CudaOps:
         scratch = torch.empty(2 * T * heads * key_dim, dtype=torch.float32, device=qk.device)
         out = torch.empty(T, heads, value_dim, dtype=torch.float32, device=qk.device)
         rot = 2 * frequencies.shape[0] if frequencies is not None else 0
+        chunk_scratch, small = self._chunk_scratch(qk.dtype, step, lambda: self.lib.pih_retention_chunk_scratch(
+            _DT[qk.dtype], _ptr(v), c_ll(v.stride(0)), T, step.num_requests, heads, key_dim, value_dim), qk.device)
         rc = self.lib.pih_retention(_DT[qk.dtype], _ptr(qk), c_ll(qk.stride(0)), _ptr(v), c_ll(v.stride(0)), _ptr(frequencies),
                                     rot, _ptr(step.positions), _ptr(decay_minus_one), c_float(key_scale), _ptr(scratch),
                                     _ptr(out), _ptr(state), c_ll(state.stride(0)), _ptr(step.cu_q), _ptr(step.state_slots),
-                                    T, step.num_requests, heads, key_dim, value_dim, self._stream())
+                                    T, step.num_requests, heads, key_dim, value_dim, _ptr(chunk_scratch), small, self._stream())
         self._check(rc, "retention")
-        self.launches += 1                                     # two kernels
+        self.launches += 1 + (2 + small if chunk_scratch is not None else 0)      # (of two to five kernels)
         return out
+
+    chunk_min_rows = 64                    # bf16 recurrences: a step whose largest request has more rows goes by chunks
+
+    def _chunk_scratch(self, dtype: torch.dtype, step, need, device):
+        """(scratch of a recurrence that goes by chunks of 64 rows or None, whether the step has requests of at most 16 rows
+        beside them).  bf16 only: in 32-bit a row's bits do not depend on where a request is cut.  A step whose largest
+        request has no more than 64 rows stays with the token loop, which 64 rows take no longer than the chunks' kernels."""
+        if dtype != torch.bfloat16 or not self.chunked_memory:
+            return None, 1
+        big, small_rows, _ = self._row_plan(step)
+        numbers = need() if big > self.chunk_min_rows else 0
+        if numbers <= 0:
+            return None, 1
+        return torch.empty(int(numbers), dtype=torch.float32, device=device), 1 if small_rows > 0 else 0
 
     def diff_qk_prepare(self, qkv: torch.Tensor, *, q_norm, k_norm, eps: float, frequencies, positions, slot_mapping,
                         cache: torch.Tensor, write_kv: bool, heads: int, kv_heads: int, key_dim: int, value_dim: int) -> None:

@@ -106,30 +106,52 @@ __device__ __forceinline__ void multiply_rows(float2 (&acc)[RM][RN], const float
   }
 }
 
-// acc[i][2 g + u] (columns 64 g + 4 tx + 2 u, + 1) += sum over k < K (a multiple of 4) of a[row][k] b[k][column].
+template <int R, int C>
+__device__ __forceinline__ void clear(float2 (&acc)[R][C]) {
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+#pragma unroll
+    for (int j = 0; j < C; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
+}
+
+// acc[i][2 g + u] (columns 64 g + 4 tx + 2 u, + 1) += sum over k < K (a multiple of 4) of a[row][k] b[k][column].  Chains of
+// 16 products, whose sums are added up: the rounding error is that of 16 + K / 16 additions, not of K.
 template <int RM, int RN>
 __device__ __forceinline__ void multiply_columns(float2 (&acc)[RM][RN / 2], const float* a, int lda, const float* b, int ldb, int K) {
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-#pragma unroll 2
-  for (int k = 0; k < K; k += 4) {
-    float4 y[4][RN / 4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int g = 0; g < RN / 4; ++g) y[u][g] = *reinterpret_cast<const float4*>(b + (k + u) * ldb + 64 * g + 4 * tx);
-#pragma unroll
-    for (int i = 0; i < RM; ++i) {
-      const float4 x = *reinterpret_cast<const float4*>(a + (ty * RM + i) * lda + k);
-      const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll 1
+  for (int k0 = 0; k0 < K; k0 += 16) {
+    float2 part[RM][RN / 2];
+    clear(part);
+    const int end = min(K, k0 + 16);
+#pragma unroll 1
+    for (int k = k0; k < end; k += 4) {
+      float4 y[4][RN / 4];
 #pragma unroll
       for (int u = 0; u < 4; ++u)
 #pragma unroll
-        for (int g = 0; g < RN / 4; ++g) {
-          const float2 xx = make_float2(xs[u], xs[u]);
-          acc[i][2 * g] = fma2(xx, make_float2(y[u][g].x, y[u][g].y), acc[i][2 * g]);
-          acc[i][2 * g + 1] = fma2(xx, make_float2(y[u][g].z, y[u][g].w), acc[i][2 * g + 1]);
-        }
+        for (int g = 0; g < RN / 4; ++g) y[u][g] = *reinterpret_cast<const float4*>(b + (k + u) * ldb + 64 * g + 4 * tx);
+#pragma unroll
+      for (int i = 0; i < RM; ++i) {
+        const float4 x = *reinterpret_cast<const float4*>(a + (ty * RM + i) * lda + k);
+        const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int g = 0; g < RN / 4; ++g) {
+            const float2 xx = make_float2(xs[u], xs[u]);
+            part[i][2 * g] = fma2(xx, make_float2(y[u][g].x, y[u][g].y), part[i][2 * g]);
+            part[i][2 * g + 1] = fma2(xx, make_float2(y[u][g].z, y[u][g].w), part[i][2 * g + 1]);
+          }
+      }
     }
+#pragma unroll
+    for (int i = 0; i < RM; ++i)
+#pragma unroll
+      for (int j = 0; j < RN / 2; ++j) {
+        acc[i][j].x += part[i][j].x;
+        acc[i][j].y += part[i][j].y;
+      }
   }
 }
 
@@ -156,14 +178,6 @@ __device__ __forceinline__ void multiply_outer(float2 (&acc)[RM][RN / 2], const 
       }
     }
   }
-}
-
-template <int R, int C>
-__device__ __forceinline__ void clear(float2 (&acc)[R][C]) {
-#pragma unroll
-  for (int i = 0; i < R; ++i)
-#pragma unroll
-    for (int j = 0; j < C; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
 }
 
 }  // namespace chunks

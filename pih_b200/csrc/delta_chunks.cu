@@ -273,22 +273,45 @@ delta_chunk_prepare_kernel(const DeltaChunkArgs p) {
   }
 }
 
-template <int DIM, int VS>
-constexpr size_t delta_states_bytes() {
-  return sizeof(float) * (2 * chunks::kRows * (DIM + 4) + 2 * chunks::kRows * DIM + 3 * chunks::kRows * VS + VS * (DIM + 4));
+// Sums over LANES neighbouring lanes of N numbers each: lane i of them keeps the N / LANES from i * N / LANES on, in v[0] ...
+template <int N, int LANES>
+__device__ __forceinline__ void sum_and_share(float (&v)[N]) {
+  const int lane = threadIdx.x & 31;
+  int n = N;
+#pragma unroll
+  for (int m = LANES / 2; m > 0; m >>= 1) {
+    n >>= 1;
+    const bool upper = lane & m;
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) {
+      if (i >= n) break;
+      const float mine = upper ? v[i + n] : v[i], other = upper ? v[i] : v[i + n];
+      v[i] = mine + __shfl_xor_sync(0xffffffffu, other, m);
+    }
+  }
 }
 
-// Block (request, head, VS value columns), 256 threads, the request's chunks in order.  A chunk's W, k and U0 are copied
-// while the chunk before is computed; bound by the chain of two products and two barriers a chunk.
-template <int DIM, int VS>
+constexpr int kValues = 8;                                 // value columns a block of delta_chunk_states
+
+template <int DIM>
+constexpr size_t delta_states_bytes() {
+  return sizeof(float) * (4 * chunks::kRows * (DIM + 4) + 2 * chunks::kRows * kValues + chunks::kRows * (kValues + 4) + kValues * (DIM + 4));
+}
+
+// Block (request, head, 8 value columns), 256 threads, the request's chunks in order.  A chunk's W, k and U0 are copied
+// while the chunk before is computed.  Both products are cut along the sum as well — a thread 4 rows by 8 columns of a
+// sixteenth (or eighth) of it, the shares met by shuffles — because a thread with whole sums of two or four outputs reads
+// three 16-byte pieces for eight products (80 us for 24 chunks of 8 heads of 128 x 128, bound by those reads; 57 us now).
+template <int DIM>
 __global__ void __launch_bounds__(256)
 delta_chunk_states_kernel(const DeltaChunkArgs p) {
-  constexpr int R = chunks::kRows, LD = DIM + 4, kStage = R * LD + R * DIM + R * VS;
-  constexpr int CU = R * VS / 256;                         // columns of U a thread (of one row)
-  constexpr int CS = DIM * VS / 256;                       // columns of S a thread (of one channel)
-  extern __shared__ __align__(16) float smem[];            // [2][W [64][LD] | k [64][DIM] | U0 [64][VS]]
-  float* us = smem + 2 * kStage;                           // [64][VS]
-  float* st = us + R * VS;                                 // [VS][LD]: S, a column after the other
+  constexpr int R = chunks::kRows, LD = DIM + 4, VS = kValues, LU = VS + 4, kStage = 2 * R * LD + R * VS;
+  constexpr int CU = R * VS / 256, USplit = 16;            // columns of U a thread ends with (of one row); lanes that share a sum
+  constexpr int CS = DIM * VS / 256, SSplit = 32 / CS;     // the same of S (of one channel)
+  static_assert(CU == 32 / USplit, "32 outputs for every group of lanes");
+  extern __shared__ __align__(16) float smem[];            // [2][W [64][LD] | k [64][LD] | U0 [64][VS]]
+  float* us = smem + 2 * kStage;                           // [64][LU]
+  float* st = us + R * LU;                                 // [VS][LD]: S, a column after the other
   __shared__ int first;
   wait_for_prior_kernels();
   launch_dependents();
@@ -307,20 +330,21 @@ delta_chunk_states_kernel(const DeltaChunkArgs p) {
     for (int e = tid; e < R * DIM / 4; e += 256) {
       const int row = e / (DIM / 4), col = (e % (DIM / 4)) * 4;
       chunks::copy_async_16(to + row * LD + col, from + at.w + row * DIM + col);
-      chunks::copy_async_16(to + R * LD + row * DIM + col, from + at.k + row * DIM + col);
+      chunks::copy_async_16(to + (R + row) * LD + col, from + at.k + row * DIM + col);
     }
     for (int e = tid; e < R * VS / 4; e += 256) {
       const int row = e / (VS / 4), col = (e % (VS / 4)) * 4;
-      chunks::copy_async_16(to + R * LD + R * DIM + row * VS + col, from + at.u + static_cast<long long>(row) * p.vdim + v0 + col);
+      chunks::copy_async_16(to + 2 * R * LD + row * VS + col, from + at.u + static_cast<long long>(row) * p.vdim + v0 + col);
     }
     chunks::copies_commit();
   };
-  const int sd = tid / (VS / CS), sc = (tid % (VS / CS)) * CS;               // this thread's numbers of S
+  // what this thread's shares of the sums end as: CS numbers of S (channel sd, columns sc ...), CU of U (row ur, columns uc ...)
+  const int sd = tid / (VS / CS), sc = (tid % (VS / CS)) * CS, ur = tid / (VS / CU), uc = (tid % (VS / CU)) * CU;
   float* Sg = p.state + slot * p.state_stride + (static_cast<long long>(h) * DIM + sd) * p.vdim + v0 + sc;
   float S[CS];
 #pragma unroll
   for (int i = 0; i < CS; ++i) S[i] = Sg[i];
-  const int ur = tid / (VS / CU), uc = (tid % (VS / CU)) * CU;               // and of U
+  const int u_tile = tid / USplit * 4, u_share = tid % USplit, s_tile = tid / SSplit * 4, s_share = tid % SSplit;
   fetch(0);
   for (int c = 0; c < count; ++c) {
 #pragma unroll
@@ -330,47 +354,67 @@ delta_chunk_states_kernel(const DeltaChunkArgs p) {
     __syncthreads();                                       // the chunk and S are there; the chunk before is done with
     if (c + 1 < count) fetch(c + 1);
     store_numbers<CS>(base + c * step + at.state + static_cast<long long>(sd) * p.vdim + v0 + sc, S);
-    const float *ws = smem + (c & 1) * kStage, *ks = ws + R * LD, *u0 = ks + R * DIM;
-    float2 sum[CU][2];
+    const float *ws = smem + (c & 1) * kStage, *ks = ws + R * LD, *u0 = ks + R * LD;
+    float sums[32];
+    {
+      float2 part[4][VS];
+      chunks::clear(part);
 #pragma unroll
-    for (int i = 0; i < CU; ++i) sum[i][0] = sum[i][1] = make_float2(0.0f, 0.0f);
-#pragma unroll 8
-    for (int e = 0; e < DIM; e += 4) {
-      const float4 w = *reinterpret_cast<const float4*>(ws + ur * LD + e);
+      for (int e = 4 * u_share; e < DIM; e += 4 * USplit) {
+        float4 s[VS];
 #pragma unroll
-      for (int i = 0; i < CU; ++i) {
-        const float4 s = *reinterpret_cast<const float4*>(st + (uc + i) * LD + e);
-        sum[i][0] = fma2(make_float2(w.x, w.y), make_float2(s.x, s.y), sum[i][0]);
-        sum[i][1] = fma2(make_float2(w.z, w.w), make_float2(s.z, s.w), sum[i][1]);
+        for (int j = 0; j < VS; ++j) s[j] = *reinterpret_cast<const float4*>(st + j * LD + e);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float4 w = *reinterpret_cast<const float4*>(ws + (u_tile + i) * LD + e);
+#pragma unroll
+          for (int j = 0; j < VS; ++j) {
+            part[i][j] = fma2(make_float2(w.x, w.y), make_float2(s[j].x, s[j].y), part[i][j]);
+            part[i][j] = fma2(make_float2(w.z, w.w), make_float2(s[j].z, s[j].w), part[i][j]);
+          }
+        }
       }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < VS; ++j) sums[i * VS + j] = part[i][j].x + part[i][j].y;
     }
+    sum_and_share<32, USplit>(sums);
     float u[CU];
     load_numbers<CU>(u, u0 + ur * VS + uc);
 #pragma unroll
-    for (int i = 0; i < CU; ++i) u[i] -= (sum[i][0].x + sum[i][1].x) + (sum[i][0].y + sum[i][1].y);
-    store_numbers<CU>(us + ur * VS + uc, u);
+    for (int i = 0; i < CU; ++i) u[i] -= sums[i];
+    store_numbers<CU>(us + ur * LU + uc, u);
     store_numbers<CU>(base + c * step + at.u + static_cast<long long>(ur) * p.vdim + v0 + uc, u);
     __syncthreads();
-    float a0[CS], a1[CS];
+    {
+      float2 part[4][VS / 2];
+      chunks::clear(part);
+#pragma unroll 4
+      for (int j = s_share; j < R; j += SSplit) {
+        const float4 k = *reinterpret_cast<const float4*>(ks + j * LD + s_tile);
+        const float4 lo = *reinterpret_cast<const float4*>(us + j * LU), hi = *reinterpret_cast<const float4*>(us + j * LU + 4);
+        const float kk[4] = {k.x, k.y, k.z, k.w};
 #pragma unroll
-    for (int i = 0; i < CS; ++i) {
-      a0[i] = 0.0f;
-      a1[i] = 0.0f;
-    }
-#pragma unroll 8
-    for (int j = 0; j < R; j += 2) {
-      const float k0 = ks[j * DIM + sd], k1 = ks[(j + 1) * DIM + sd];
-      float u0[CS], u1[CS];
-      load_numbers<CS>(u0, us + j * VS + sc);
-      load_numbers<CS>(u1, us + (j + 1) * VS + sc);
-#pragma unroll
-      for (int i = 0; i < CS; ++i) {
-        a0[i] = fmaf(k0, u0[i], a0[i]);
-        a1[i] = fmaf(k1, u1[i], a1[i]);
+        for (int i = 0; i < 4; ++i) {
+          const float2 f = make_float2(kk[i], kk[i]);
+          part[i][0] = fma2(f, make_float2(lo.x, lo.y), part[i][0]);
+          part[i][1] = fma2(f, make_float2(lo.z, lo.w), part[i][1]);
+          part[i][2] = fma2(f, make_float2(hi.x, hi.y), part[i][2]);
+          part[i][3] = fma2(f, make_float2(hi.z, hi.w), part[i][3]);
+        }
       }
-    }
 #pragma unroll
-    for (int i = 0; i < CS; ++i) S[i] = fmaf(end, S[i], a0[i] + a1[i]);
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < VS / 2; ++j) {
+          sums[i * VS + 2 * j] = part[i][j].x;
+          sums[i * VS + 2 * j + 1] = part[i][j].y;
+        }
+    }
+    sum_and_share<32, SSplit>(sums);
+#pragma unroll
+    for (int i = 0; i < CS; ++i) S[i] = fmaf(end, S[i], sums[i]);
   }
 #pragma unroll
   for (int i = 0; i < CS; ++i) Sg[i] = S[i];
@@ -443,10 +487,10 @@ static void allow_shared(K kernel, size_t bytes) {
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
 }
 
-template <int DIM, int VS>
+template <int DIM>
 static void launch_states(cudaStream_t s, const DeltaChunkArgs& p) {
-  allow_shared(delta_chunk_states_kernel<DIM, VS>, delta_states_bytes<DIM, VS>());
-  launch_kernel(delta_chunk_states_kernel<DIM, VS>, dim3(p.requests, p.heads, p.vdim / VS), dim3(256), delta_states_bytes<DIM, VS>(), s, p);
+  allow_shared(delta_chunk_states_kernel<DIM>, delta_states_bytes<DIM>());
+  launch_kernel(delta_chunk_states_kernel<DIM>, dim3(p.requests, p.heads, p.vdim / kValues), dim3(256), delta_states_bytes<DIM>(), s, p);
 }
 template <int DIM, int VT>
 static void launch_out(cudaStream_t s, const DeltaChunkArgs& p, unsigned count) {
@@ -459,9 +503,7 @@ static int launch_chunks(cudaStream_t s, const DeltaChunkArgs& p, int rows) {
   allow_shared(delta_chunk_prepare_kernel<DIM, CHANNELS>, delta_prepare_bytes<DIM>());
   launch_kernel(delta_chunk_prepare_kernel<DIM, CHANNELS>, dim3(count, p.heads), dim3(256), delta_prepare_bytes<DIM>(), s, p);
   PIH_LAUNCH_CHECK();
-  // 8 value columns a block where every block then has an SM of its own; else 16, in fewer rounds
-  if (static_cast<long long>(p.requests) * p.heads * (p.vdim / 8) <= 148) launch_states<DIM, 8>(s, p);
-  else launch_states<DIM, 16>(s, p);
+  launch_states<DIM>(s, p);
   PIH_LAUNCH_CHECK();
   if (p.vdim % 128 == 0) launch_out<DIM, 128>(s, p, count);
   else launch_out<DIM, 64>(s, p, count);

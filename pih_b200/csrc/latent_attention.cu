@@ -15,6 +15,7 @@
 //   latent_attention_split    a block a (row, part of its keys, 8 heads) and a merge: bf16, any rank
 //   latent_attention_mma      the same cut on tensor cores (the heads are the rows of the MMA): bf16, rank 64 .. 512
 #include "common.cuh"
+#include "mma.cuh"
 
 namespace pih {
 
@@ -275,12 +276,18 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 }
 
 constexpr int kMmaTileKeys = 128;
+constexpr int latent_buffers(int rank, int rows_per_block) { return rows_per_block == 4 && rank <= 256 ? 2 : 1; }
 
 // kRowsPerBlock = 1: the block is one row (blockIdx.x), its 8 warps take the tile's 8 groups of 16 keys.
 // kRowsPerBlock = 4: the block is 4 consecutive rows of ONE request (blockIdx.x counts the requests' row tiles, found
 // by walking cu_q; blocks beyond the last tile leave), so a tile of latents is fetched once for 4 rows: warp w is row
 // w % 4 and takes every second group of 16 keys.  Parts a (row, head): splits * 8 / kRowsPerBlock.
-template <int kRank, int kOut, int kRowsPerBlock>
+// kPack = 2 (with kRowsPerBlock = 4): at most 8 heads, whose other 8 rows of the MMA would be empty: a warp holds two
+// consecutive rows, 8 heads each, and the block 8 rows, so that both the products and the tiles serve twice the rows.
+// A prompt's blocks (one on an SM, for their registers) copy the next tile while they compute on this one, where two fit;
+// the sums are rescaled only where a maximum of the warp has moved (2048 rows of 8 heads of rank 256 and a window of 1024:
+// 321 us without the three, 138 us with them).
+template <int kRank, int kOut, int kRowsPerBlock, int kPack>
 __global__ void __launch_bounds__(256)
 latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache,
                             const int* __restrict__ block_table, int table_width, const int* __restrict__ request_of_row,
@@ -290,14 +297,16 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
   typedef __nv_bfloat16 bf;
   constexpr int kPitch = kRank + 8;                              // elements; rows 16 bytes apart in the banks
   constexpr int kStreams = 8 / kRowsPerBlock;                    // warps a row, each a stream of its own over keys
+  constexpr int kRows = kRowsPerBlock * kPack;                   // rows of the block
+  constexpr int kBuffers = latent_buffers(kRank, kRowsPerBlock);
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ long long src_row[kMmaTileKeys];
+  __shared__ long long src_rows[kBuffers][kMmaTileKeys];
   wait_for_prior_kernels();
   launch_dependents();
   // a latent wider than 256: the block computes every score but only kOut of the sum's columns (the accumulators of
   // all of them would not fit a thread's registers); blockIdx.z counts (group of heads, stretch of columns)
   constexpr int kStretches = kRank / kOut;
-  const int split = blockIdx.y, h0 = (blockIdx.z / kStretches) * 16;
+  const int split = blockIdx.y, h0 = (blockIdx.z / kStretches) * (16 / kPack);
   const int cbase = (blockIdx.z % kStretches) * kOut;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t4 = lane & 3;
@@ -311,16 +320,16 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
     int b = blockIdx.x;
     req = 0;
     for (; req < requests; ++req) {
-      const int tiles = (cu_q[req + 1] - cu_q[req] + kRowsPerBlock - 1) / kRowsPerBlock;
+      const int tiles = (cu_q[req + 1] - cu_q[req] + kRows - 1) / kRows;
       if (b < tiles) break;
       b -= tiles;
     }
     if (req >= requests) return;                                 // beyond the last row tile
-    row0 = cu_q[req] + b * kRowsPerBlock;
-    n_rows = min(kRowsPerBlock, cu_q[req + 1] - row0);
+    row0 = cu_q[req] + b * kRows;
+    n_rows = min(kRows, cu_q[req + 1] - row0);
   }
   bf* Qs = reinterpret_cast<bf*>(smem_raw);                      // [kRowsPerBlock * 16][kPitch]
-  bf* tile = Qs + kRowsPerBlock * 16 * kPitch;                   // [128][kPitch]
+  bf* tiles = Qs + kRowsPerBlock * 16 * kPitch;                  // [kBuffers][128][kPitch]
   // the block's keys: from the first row's first key to the last row's position, cut into ``splits``
   const int pos_last = positions[row0 + n_rows - 1];
   const int first_0 = window > 0 ? max(0, positions[row0] - window + 1) : 0;
@@ -329,45 +338,71 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
   constexpr int kUnits = kRank / 8;                              // 16-byte units a row
   for (int i = tid; i < kRowsPerBlock * 16 * kUnits; i += 256) {
     const int rr = i / kUnits, un = i - rr * kUnits;
-    const int ri = rr / 16, hh = rr % 16;
+    const int ri = rr / (16 / kPack), hh = rr % (16 / kPack);
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     if (ri < n_rows && h0 + hh < heads)
       v = *reinterpret_cast<const uint4*>(q + (static_cast<long long>(row0 + ri) * heads + h0 + hh) * kRank + un * 8);
     *reinterpret_cast<uint4*>(Qs + rr * kPitch + un * 8) = v;
   }
-  // this warp's row and its share of a tile's groups of 16 keys
+  // this warp's row (rows: of the upper and the lower half of the MMA's) and its share of a tile's groups of 16 keys
   const int ri = warp % kRowsPerBlock, stream = warp / kRowsPerBlock;
-  const bool active = ri < n_rows;
-  const int pos = active ? positions[row0 + ri] : -1;
-  const int first = (active && window > 0) ? max(0, pos - window + 1) : 0;
+  const int ra = ri * kPack, rb = ra + kPack - 1;
+  const bool active = ra < n_rows;
+  const int pos_a = active ? positions[row0 + ra] : -1, pos_b = rb < n_rows ? positions[row0 + rb] : -1;
+  const int first_a = (active && window > 0) ? max(0, pos_a - window + 1) : 0;
+  const int first_b = (rb < n_rows && window > 0) ? max(0, pos_b - window + 1) : 0;
+  const int pos = max(pos_a, pos_b), first = first_a;            // what any of them sees
   float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.0f, l1 = 0.0f;
   float O[kOut / 8][4];
 #pragma unroll
   for (int n = 0; n < kOut / 8; ++n) { O[n][0] = O[n][1] = O[n][2] = O[n][3] = 0.0f; }
   const int* table = block_table + static_cast<long long>(req) * table_width;
   const int mi = lane >> 3, lr = lane & 7;
-  for (int t0 = k0; t0 < k1; t0 += kMmaTileKeys) {
-    __syncthreads();                                             // the tile before this one has been used
-    if (tid < kMmaTileKeys) {
-      const int key = t0 + tid;
-      long long src = -1;
-      if (key < k1) {
-        const int pi = key / page_size;
-        const int page = pi < table_width ? table[pi] : -1;
-        if (page < 0 || page >= num_pages) publish_error(err, kRowWithoutPage);
-        else src = (static_cast<long long>(page) * page_size + (key - pi * page_size)) * kRank;
-      }
-      src_row[tid] = src;
+  auto find = [&](int t0, int buffer) {                          // where the tile's keys lie
+    if (tid >= kMmaTileKeys) return;
+    const int key = t0 + tid;
+    long long src = -1;
+    if (key < k1) {
+      const int pi = key / page_size;
+      const int page = pi < table_width ? table[pi] : -1;
+      if (page < 0 || page >= num_pages) publish_error(err, kRowWithoutPage);
+      else src = (static_cast<long long>(page) * page_size + (key - pi * page_size)) * kRank;
     }
-    __syncthreads();
+    src_rows[buffer][tid] = src;
+  };
+  auto fetch = [&](int buffer) {
+    bf* to = tiles + buffer * kMmaTileKeys * kPitch;
     for (int i = tid; i < kMmaTileKeys * kUnits; i += 256) {
       const int j = i / kUnits, un = i - j * kUnits;
-      const long long src = src_row[j];
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (src >= 0) v = *reinterpret_cast<const uint4*>(cache + src + un * 8);
-      *reinterpret_cast<uint4*>(tile + j * kPitch + un * 8) = v;
+      const long long src = src_rows[buffer][j];
+      if (src >= 0) mma::copy_async_16(to + j * kPitch + un * 8, cache + src + un * 8);
+      else *reinterpret_cast<uint4*>(to + j * kPitch + un * 8) = make_uint4(0u, 0u, 0u, 0u);
     }
+    mma::copy_async_commit();
+  };
+  if (kBuffers == 2 && k0 < k1) {
+    find(k0, 0);
     __syncthreads();
+    fetch(0);
+  }
+  int buffer = 0;
+  for (int t0 = k0; t0 < k1; t0 += kMmaTileKeys) {
+    if (kBuffers == 2) {
+      buffer = ((t0 - k0) / kMmaTileKeys) & 1;
+      if (t0 + kMmaTileKeys < k1) find(t0 + kMmaTileKeys, buffer ^ 1);
+      mma::copy_async_wait<0>();
+      __syncthreads();                                           // this tile is there, the one before it has been used
+      if (t0 + kMmaTileKeys < k1) fetch(buffer ^ 1);
+    } else {
+      __syncthreads();                                           // the tile before this one has been used
+      find(t0, 0);
+      __syncthreads();
+      fetch(0);
+      mma::copy_async_wait<0>();
+      __syncthreads();
+    }
+    const bf* tile = tiles + buffer * kMmaTileKeys * kPitch;
+    const long long* src_row = src_rows[buffer];
     if (!active) continue;
     for (int kl = stream * 16; kl < kMmaTileKeys; kl += kStreams * 16) {      // this warp's keys within the tile
       if (t0 + kl >= k1 || t0 + kl > pos || t0 + kl + 15 < first) continue;
@@ -387,7 +422,8 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
         for (int c = 0; c < 4; ++c) {
           const int kk = kl + nt * 8 + 2 * t4 + (c & 1);
           const int key = t0 + kk;
-          const bool valid = key < k1 && key <= pos && key >= first && src_row[kk] >= 0;
+          const bool valid = key < k1 && key <= (c < 2 ? pos_a : (kPack == 2 ? pos_b : pos_a)) &&
+                             key >= (c < 2 ? first_a : (kPack == 2 ? first_b : first_a)) && src_row[kk] >= 0;
           S[nt][c] = valid ? S[nt][c] * scale : -INFINITY;
           if (c < 2) mx0 = fmaxf(mx0, S[nt][c]); else mx1 = fmaxf(mx1, S[nt][c]);
         }
@@ -420,16 +456,16 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
       pa[1] = pack_bf16(S[0][2], S[0][3]);
       pa[2] = pack_bf16(S[1][0], S[1][1]);
       pa[3] = pack_bf16(S[1][2], S[1][3]);
+      if (__any_sync(0xffffffffu, corr0 != 1.0f || corr1 != 1.0f)) {
+#pragma unroll
+        for (int n = 0; n < kOut / 8; ++n) { O[n][0] *= corr0; O[n][1] *= corr0; O[n][2] *= corr1; O[n][3] *= corr1; }
+      }
 #pragma unroll
       for (int nb = 0; nb < kOut / 16; ++nb) {
         uint32_t b[4];
         ldmatrix_x4_trans(b, tile + (kl + lr + (mi & 1) * 8) * kPitch + cbase + nb * 16 + (mi >> 1) * 8);
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          float (&o)[4] = O[2 * nb + half];
-          o[0] *= corr0; o[1] *= corr0; o[2] *= corr1; o[3] *= corr1;
-          mma_bf16(o, pa, b[2 * half], b[2 * half + 1]);
-        }
+        mma_bf16(O[2 * nb], pa, b[0], b[1]);
+        mma_bf16(O[2 * nb + 1], pa, b[2], b[3]);
       }
     }
   }
@@ -437,9 +473,9 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
   const int parts = splits * kStreams;
 #pragma unroll
   for (int hr = 0; hr < 2; ++hr) {
-    const int h = h0 + g + hr * 8;
-    if (h >= heads) continue;
-    float* dst = partial + ((static_cast<long long>(row0 + ri) * heads + h) * parts + split * kStreams + stream) * (kRank + 2);
+    const int h = h0 + g + (kPack == 2 ? 0 : hr * 8), row = ra + (kPack == 2 ? hr : 0);
+    if (h >= heads || row >= n_rows) continue;
+    float* dst = partial + ((static_cast<long long>(row0 + row) * heads + h) * parts + split * kStreams + stream) * (kRank + 2);
     if (t4 == 0 && cbase == 0) { dst[0] = hr ? m1 : m0; dst[1] = hr ? l1 : l0; }
 #pragma unroll
     for (int n = 0; n < kOut / 8; ++n) {
@@ -626,9 +662,9 @@ extern "C" int pih_latent_attention_split(int dtype, const void* q, const void* 
   return 0;
 }
 
-// The tensor-core kernel: bf16, rank 64, 128, 192, 256, 384 or 512.  rows_per_block 1 or 4 (4: blocks are row tiles
-// of a request, for steps of prompt portions).  partial: fp32 scratch, rows * heads * parts * (rank + 2) with
-// parts = splits * 8 / rows_per_block.
+// The tensor-core kernel: bf16, rank 64, 128, 192, 256, 384 or 512.  rows_per_block 1, 4 or (at most 8 heads) 8; 4 and 8:
+// blocks are row tiles of a request, for steps of prompt portions.  partial: fp32 scratch, rows * heads * parts * (rank + 2)
+// with parts = splits * 8 for 1, else splits * 2.
 extern "C" int pih_latent_attention_mma(const void* q, const void* gate, long long ldg, const void* sink, const void* cache,
                                         const void* block_table, int table_width, const void* request_of_row,
                                         const void* positions, const void* cu_q, int requests, void* partial, void* out,
@@ -636,19 +672,21 @@ extern "C" int pih_latent_attention_mma(const void* q, const void* gate, long lo
                                         int window, int splits, int rows_per_block, void* err, void* stream) {
   if (rows <= 0) return 0;
   if ((rank != 64 && rank != 128 && rank != 192 && rank != 256 && rank != 384 && rank != 512) || splits < 1 ||
-      (rows_per_block != 1 && rows_per_block != 4) || splits * 8 / rows_per_block > kMergeParts || rows > 65535 * 32)
+      (rows_per_block != 1 && rows_per_block != 4 && (rows_per_block != 8 || heads > 8)) ||
+      splits * (rows_per_block == 1 ? 8 : 2) > kMergeParts || rows > 65535 * 32)
     return PIH_ERR_UNSUPPORTED;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const size_t smem = (16 * rows_per_block + kMmaTileKeys) * static_cast<size_t>(rank + 8) * 2;
-  const unsigned blocks_x = rows_per_block == 1 ? rows : (rows + 3) / 4 + requests;
+  const int q_rows = 16 * min(rows_per_block, 4), buffers = latent_buffers(rank, min(rows_per_block, 4));
+  const size_t smem = (q_rows + buffers * kMmaTileKeys) * static_cast<size_t>(rank + 8) * 2;
+  const unsigned blocks_x = rows_per_block == 1 ? rows : (rows + rows_per_block - 1) / rows_per_block + requests;
   dim3 grid(blocks_x, splits, (heads + 15) / 16 * (rank > 256 ? 2 : 1));
   const long long items = static_cast<long long>(rows) * heads;
-#define PIH_LM1(R, C, B)                                                                                               \
+#define PIH_LM1(R, C, B, K)                                                                                             \
   do {                                                                                                                 \
     if (smem > 48 * 1024)                                                                                              \
-      cudaFuncSetAttribute(latent_attention_mma_kernel<R, C, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,          \
+      cudaFuncSetAttribute(latent_attention_mma_kernel<R, C, B, K>, cudaFuncAttributeMaxDynamicSharedMemorySize,          \
                            static_cast<int>(smem));                                                                    \
-    launch_kernel(latent_attention_mma_kernel<R, C, B>, grid, dim3(256), smem, s, static_cast<const bf16*>(q),         \
+    launch_kernel(latent_attention_mma_kernel<R, C, B, K>, grid, dim3(256), smem, s, static_cast<const bf16*>(q),         \
                   static_cast<const bf16*>(cache), static_cast<const int*>(block_table), table_width,                  \
                   static_cast<const int*>(request_of_row), static_cast<const int*>(positions),                         \
                   static_cast<const int*>(cu_q), requests, static_cast<float*>(partial), heads, page_size, num_pages,  \
@@ -656,7 +694,9 @@ extern "C" int pih_latent_attention_mma(const void* q, const void* gate, long lo
   } while (0)
 #define PIH_LM(R, C)                                                                                                   \
   do {                                                                                                                 \
-    if (rows_per_block == 1) PIH_LM1(R, C, 1); else PIH_LM1(R, C, 4);                                                  \
+    if (rows_per_block == 1) PIH_LM1(R, C, 1, 1);                                                                      \
+    else if (rows_per_block == 4) PIH_LM1(R, C, 4, 1);                                                                 \
+    else PIH_LM1(R, C, 4, 2);                                                                                          \
   } while (0)
   if (rank == 64) PIH_LM(64, 64);
   else if (rank == 128) PIH_LM(128, 128);
@@ -670,7 +710,7 @@ extern "C" int pih_latent_attention_mma(const void* q, const void* gate, long lo
   launch_kernel(latent_merge_kernel<bf16>, dim3(static_cast<unsigned>(items)), dim3(rank >= 256 ? 256 : (rank + 31) / 32 * 32), 0, s,
                 static_cast<const float*>(partial), static_cast<const bf16*>(gate), ldg, static_cast<const float*>(sink),
                 static_cast<const int*>(request_of_row), static_cast<bf16*>(out), rows, heads, rank,
-                splits * 8 / rows_per_block, static_cast<uint32_t*>(err));
+                splits * (rows_per_block == 1 ? 8 : 2), static_cast<uint32_t*>(err));
   PIH_LAUNCH_CHECK();
   return 0;
 }

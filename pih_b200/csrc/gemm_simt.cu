@@ -3,8 +3,8 @@
 // This is the matrix product of the true 32-bit path (no tensor cores, no
 // TF32, no split tricks) and the plain twin of the tensor-core products.  It
 // also takes bf16 inputs and writes bf16 or fp32.  Every output element is
-// accumulated by one thread in ascending k — sixteen products into a partial
-// sum, the partial sums into the total, which keeps the rounding error of a
+// accumulated in an order that k alone decides — short chains into partial
+// sums, the partial sums into the total, which keeps the rounding error of a
 // long sum (k of a thousand and more) near that of a short one — so a row's
 // result does not depend on how many other rows the call holds: cutting a
 // prompt into portions or batching it with other requests cannot change a bit.

@@ -12,7 +12,7 @@ def ops():
 
 
 def _bound(x, w):
-    # a chain of 32 products, half a dozen partial sums of 64 and at most eight slices: every product meets fewer than 64
+    # a chain of 16 products, at most a dozen tiles of 32 in a slice and eight slices: every product meets fewer than 64
     # roundings of 2^-24 of a sum that is at most the sum of the magnitudes
     return 64 * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
 

@@ -96,8 +96,8 @@ gemm_simt_kernel(const TA* __restrict__ A, const TA* __restrict__ W, TC* __restr
 //     innermost: a 16-byte read of an operand is two pairs of neighbouring k for the two-number FMA.  Rows of 36 words
 //     put the 16-byte reads of eight neighbouring rows into different banks.
 //   * An output's even and odd products of a tile run in two chains of 16, whose sum joins the slice's: closer to the exact
-//     sum than the 16 products and K / 16 partial sums above for short and long k alike.  (Chains of 32 are 3 % faster, and
-//     further off for k of a hundred.)
+//     sum than the 16 products and K / 16 partial sums above for short and long k alike.  (Chains of 32 were no
+//     faster, and further off for k of a hundred.)
 // Tiles of 8 x 64 for at most 8 rows, 32 x 64 up to 32, 64 x 64 beyond: a wider tile would only add rows of padding.
 constexpr int kTileK = 32, kTileLd = kTileK + 4, kTileN = 64, kTileThreads = 128;
 

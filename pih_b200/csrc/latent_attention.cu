@@ -285,8 +285,8 @@ constexpr int latent_buffers(int rank, int rows_per_block) { return rows_per_blo
 // kPack = 2 (with kRowsPerBlock = 4): at most 8 heads, whose other 8 rows of the MMA would be empty: a warp holds two
 // consecutive rows, 8 heads each, and the block 8 rows, so that both the products and the tiles serve twice the rows.
 // A prompt's blocks (one on an SM, for their registers) copy the next tile while they compute on this one, where two fit;
-// the sums are rescaled only where a maximum of the warp has moved (2048 rows of 8 heads of rank 256 and a window of 1024:
-// 321 us without the three, 138 us with them).
+// the sums are rescaled only where a maximum of the warp has moved (2048 rows of 8 heads of rank 256 and a window of 1024,
+// with the merge: 349 us without the three, 172 us with them).
 template <int kRank, int kOut, int kRowsPerBlock, int kPack>
 __global__ void __launch_bounds__(256)
 latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache,
@@ -300,7 +300,10 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
   constexpr int kRows = kRowsPerBlock * kPack;                   // rows of the block
   constexpr int kBuffers = latent_buffers(kRank, kRowsPerBlock);
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ long long src_rows[kBuffers][kMmaTileKeys];
+  // the places of a tile's keys, one slot more than buffers: a tile's are written in front of the barrier that ends the tile
+  // before it, which slower warps still mask by its own
+  constexpr int kSlots = kBuffers == 2 ? 3 : 1;
+  __shared__ long long src_rows[kSlots][kMmaTileKeys];
   wait_for_prior_kernels();
   launch_dependents();
   // a latent wider than 256: the block computes every score but only kOut of the sum's columns (the accumulators of
@@ -358,7 +361,7 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
   for (int n = 0; n < kOut / 8; ++n) { O[n][0] = O[n][1] = O[n][2] = O[n][3] = 0.0f; }
   const int* table = block_table + static_cast<long long>(req) * table_width;
   const int mi = lane >> 3, lr = lane & 7;
-  auto find = [&](int t0, int buffer) {                          // where the tile's keys lie
+  auto find = [&](int t0, int slot) {                            // where the tile's keys lie
     if (tid >= kMmaTileKeys) return;
     const int key = t0 + tid;
     long long src = -1;
@@ -368,13 +371,13 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
       if (page < 0 || page >= num_pages) publish_error(err, kRowWithoutPage);
       else src = (static_cast<long long>(page) * page_size + (key - pi * page_size)) * kRank;
     }
-    src_rows[buffer][tid] = src;
+    src_rows[slot][tid] = src;
   };
-  auto fetch = [&](int buffer) {
+  auto fetch = [&](int slot, int buffer) {
     bf* to = tiles + buffer * kMmaTileKeys * kPitch;
     for (int i = tid; i < kMmaTileKeys * kUnits; i += 256) {
       const int j = i / kUnits, un = i - j * kUnits;
-      const long long src = src_rows[buffer][j];
+      const long long src = src_rows[slot][j];
       if (src >= 0) mma::copy_async_16(to + j * kPitch + un * 8, cache + src + un * 8);
       else *reinterpret_cast<uint4*>(to + j * kPitch + un * 8) = make_uint4(0u, 0u, 0u, 0u);
     }
@@ -383,26 +386,28 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
   if (kBuffers == 2 && k0 < k1) {
     find(k0, 0);
     __syncthreads();
-    fetch(0);
+    fetch(0, 0);
   }
-  int buffer = 0;
+  int buffer = 0, slot = 0;
   for (int t0 = k0; t0 < k1; t0 += kMmaTileKeys) {
     if (kBuffers == 2) {
-      buffer = ((t0 - k0) / kMmaTileKeys) & 1;
-      if (t0 + kMmaTileKeys < k1) find(t0 + kMmaTileKeys, buffer ^ 1);
+      const int number = (t0 - k0) / kMmaTileKeys, next = (number + 1) % kSlots;
+      buffer = number & 1;
+      slot = number % kSlots;
+      if (t0 + kMmaTileKeys < k1) find(t0 + kMmaTileKeys, next);
       mma::copy_async_wait<0>();
       __syncthreads();                                           // this tile is there, the one before it has been used
-      if (t0 + kMmaTileKeys < k1) fetch(buffer ^ 1);
+      if (t0 + kMmaTileKeys < k1) fetch(next, buffer ^ 1);
     } else {
       __syncthreads();                                           // the tile before this one has been used
       find(t0, 0);
       __syncthreads();
-      fetch(0);
+      fetch(0, 0);
       mma::copy_async_wait<0>();
       __syncthreads();
     }
     const bf* tile = tiles + buffer * kMmaTileKeys * kPitch;
-    const long long* src_row = src_rows[buffer];
+    const long long* src_row = src_rows[slot];
     if (!active) continue;
     for (int kl = stream * 16; kl < kMmaTileKeys; kl += kStreams * 16) {      // this warp's keys within the tile
       if (t0 + kl >= k1 || t0 + kl > pos || t0 + kl + 15 < first) continue;

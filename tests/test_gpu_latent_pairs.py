@@ -1,12 +1,59 @@
 """Portions of prompts on the latent attention's tensor-core kernel: two rows an MMA (at most 8 heads), tiles copied ahead,
 against the plain softmax."""
 import pytest
+import torch
 
 import test_gpu_rigotar as rigotar
+from test_gpu_rigotar import DEV
 
 pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("rank, heads", [(256, 8), (256, 7), (192, 1), (512, 8), (64, 8), (256, 9), (256, 16)])
 def test_portions_of_several_requests(rank, heads):
+    """Blocks of one tile each (contexts of up to 371 keys in 5 to 10 splits)."""
     rigotar.test_latent_attention_portions_of_several_requests(rank, heads)
+
+
+def _plain_windowed(q, lat, positions, window, scale):
+    """q [T, heads, rank] over latents [n, rank], float64 on the GPU."""
+    at = torch.arange(lat.shape[0], device=DEV)
+    hidden = at[None] > positions[:, None]
+    if window:
+        hidden |= at[None] <= positions[:, None] - window
+    out = torch.empty_like(q)
+    for h in range(q.shape[1]):
+        out[:, h] = torch.softmax((q[:, h] @ lat.T * scale).masked_fill(hidden, float("-inf")), -1) @ lat
+    return out
+
+
+# 1500 to 1507 rows: one split, a block's tiles are 9 with the window and up to 12 without.  301 rows behind 3700: without a
+# window 7 splits of 5 tiles (8 rows a block) or 3 of 11 (4 rows), with it 2 and 3 tiles.  The last one is seldom whole.
+@pytest.mark.parametrize("window", [0, 1024])
+@pytest.mark.parametrize("rank, heads", [(64, 8), (128, 7), (192, 8), (256, 8), (256, 16)])
+@pytest.mark.parametrize("past, rows", [(0, n) for n in range(1500, 1508)] + [(3700, 301)])
+def test_contexts_of_many_tiles(past, rows, rank, heads, window):
+    """Rows of a request over more tiles than there are buffers, all remainders of rows in the last block: its warps without
+    a row run ahead of the others, which must still see every key of their tile.  16 lost keys of 1024 are an eighth of a row."""
+    from pih_b200.kernels import get_ops
+    ops = get_ops(torch.device(DEV))
+    g = torch.Generator().manual_seed(rank + rows)
+    n, page = past + rows, 64
+    lat = (torch.randn(n, rank, generator=g) * 0.5).bfloat16().to(DEV)
+    q = (torch.randn(rows, heads, rank, generator=g) * 0.6).bfloat16().to(DEV)
+    pages = -(-n // page)
+    order = torch.randperm(pages, generator=g)
+    cache = torch.zeros(pages, page, rank, dtype=torch.bfloat16, device=DEV)
+    padded = torch.zeros(pages * page, rank, dtype=torch.bfloat16, device=DEV)
+    padded[:n] = lat
+    cache[order.to(DEV)] = padded.view(pages, page, rank)
+    positions = list(range(past, n))
+    step = rigotar._step(positions, [0] * rows, [0, rows], [0])
+    scale = rank ** -0.5
+    got = ops.latent_attention(q, gate=None, sink=None, cache=cache, block_table=order.int().to(DEV).view(1, -1), step=step,
+                               scale=scale, window=window).double()
+    ops.check_errors()
+    ref = _plain_windowed(q.double(), lat.double(), torch.tensor(positions, device=DEV), window, scale)
+    # the weights are rounded to 8 bits each (2^-9 of a term, in random directions), the output too
+    worst = float(((got - ref).norm(dim=-1) / ref.norm(dim=-1)).max())
+    assert worst < 1.5e-2, worst

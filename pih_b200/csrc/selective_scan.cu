@@ -17,13 +17,6 @@
 // State, step sizes, exponentials and sums are 32-bit.  The 32-bit path forms exp(dt A) S as S + expm1(dt A) S, so that a
 // state that remembers long keeps the distance of its decay from one; the bf16 path takes the special-function unit's 2^x.
 // The order of additions of a row does not depend on the row's place in its chunk, so a cut of the prompt changes nothing.
-//
-// bf16, a step with a request of more than 512 rows: the rows of a request follow one another on 128 threads an SM, and the
-// chain, not the arithmetic, is what a prompt costs (86 us for 1531 rows of 2048 channels of 16 states).  Such a step goes by
-// stretches of 256 rows side by side, in two launches: what every stretch but the last makes of a state of zeros, and the sum
-// of its step sizes (whose product with A is the log of its decay); then every stretch folds those of the ones in front of
-// it into the state that the request came with, and runs as above.  From 512 rows on two chains of 256 take no longer than
-// one of the whole.
 #include "common.cuh"
 #include "mma.cuh"
 
@@ -51,15 +44,7 @@ struct ScanArgs {
   const int* cu_q;
   const int* state_slots;
   int inner, states;
-  // by stretches
-  int requests;
-  float* ends;                              // [stretches][inner][states]: the state that a stretch makes of zeros
-  float* sums;                              // [stretches][inner]: its step sizes' sum
-  float* starts;                            // [requests][inner][states]: the states before the step
 };
-
-constexpr int kStretchRows = 256;
-enum ScanKind : int { kWhole = 0, kEnds = 1, kStretches = 2 };
 
 // v[0 .. COUNT-1]: a lane's shares of COUNT rows.  Afterwards v[0 .. max(1, COUNT / 2^steps)-1] are whole sums (over the lanes
 // that differ in the bits of MASK and below) of the rows from the returned one on.
@@ -88,7 +73,7 @@ struct ScanShape {
   static constexpr int kThreads = CH * kParts;
 };
 
-template <typename T, int kParts, int kN, int KIND>
+template <typename T, int kParts, int kN>
 __global__ void __launch_bounds__(ScanShape<kParts>::kThreads)
 selective_scan_kernel(const ScanArgs p) {
   constexpr bool kExact = sizeof(T) == 4;
@@ -106,20 +91,8 @@ selective_scan_kernel(const ScanArgs p) {
   Outputs y_s = reinterpret_cast<Outputs>(scan_smem + kScanRows * (2 * NP + 2 * CH));       // [rows][CH]
   wait_for_prior_kernels();
   launch_dependents();
-  const int c0 = blockIdx.y * CH, tid = threadIdx.x;
-  int r = blockIdx.x, before = 0, stretches = 1;                        // stretches of the request, and in front of this one
-  if (KIND != kWhole) {
-    int x = blockIdx.x;
-    for (r = 0; r < p.requests; ++r) {
-      stretches = (p.cu_q[r + 1] - p.cu_q[r] + kStretchRows - 1) / kStretchRows;
-      if (x < stretches) break;
-      x -= stretches;
-    }
-    if (r >= p.requests || (KIND == kEnds && x + 1 >= stretches)) return;    // (nothing comes behind a last stretch)
-    before = x;
-  }
-  const int slot = p.state_slots[r], lo = p.cu_q[r] + before * kStretchRows;
-  const int hi = KIND == kWhole ? p.cu_q[r + 1] : min(p.cu_q[r + 1], lo + kStretchRows);
+  const int r = blockIdx.x, c0 = blockIdx.y * CH, tid = threadIdx.x;
+  const int lo = p.cu_q[r], hi = p.cu_q[r + 1], slot = p.state_slots[r];
   if (hi <= lo || slot < 0) return;
   const T* u = static_cast<const T*>(p.u);
   const T* bc = static_cast<const T*>(p.bc);
@@ -134,26 +107,6 @@ selective_scan_kernel(const ScanArgs p) {
     const bool there = live && n0 + i < p.states;
     S[i] = there ? Sg[n0 + i] : 0.0f;
     A[i] = there ? p.A[static_cast<long long>(c) * p.states + n0 + i] * (kExact ? 1.0f : 1.4426950408889634f) : 0.0f;
-  }
-  const long long record = static_cast<long long>(p.inner) * p.states, mine = static_cast<long long>(c) * p.states + n0;
-  float sum = 0.0f;                                                     // kEnds: of the channel's step sizes
-  if (KIND == kEnds) {
-#pragma unroll
-    for (int i = 0; i < kN; ++i) {
-      if (before == 0 && live && n0 + i < p.states) p.starts[r * record + mine + i] = S[i];
-      S[i] = 0.0f;
-    }
-  }
-  if (KIND == kStretches && stretches > 1) {                            // (the slot is the last stretch's to write)
-#pragma unroll
-    for (int i = 0; i < kN; ++i) S[i] = live && n0 + i < p.states ? p.starts[r * record + mine + i] : 0.0f;
-    for (int b = 0; b < before && live; ++b) {
-      const long long at = static_cast<long long>(blockIdx.x) - before + b;
-      const float dt = p.sums[at * p.inner + c];
-#pragma unroll
-      for (int i = 0; i < kN; ++i)
-        if (n0 + i < p.states) S[i] = fmaf(mma::exp2_fast(dt * A[i]), S[i], p.ends[at * record + mine + i]);
-    }
   }
   // pair e of this thread: row (tid + e TH) / CH of the chunk, channel (tid + e TH) % CH of the block
   float bias[E], skip[E];
@@ -173,7 +126,7 @@ selective_scan_kernel(const ScanArgs p) {
       const int idx = tid + e * TH, t = t0 + idx / CH, ce = c0 + idx % CH;
       const bool there = idx < kScanRows * CH && t < hi && ce < p.inner;
       nx[e] = there ? u[t * p.ldu + ce] : zero;
-      nz[e] = KIND != kEnds && there ? z[t * p.ldz + ce] : zero;
+      nz[e] = there ? z[t * p.ldz + ce] : zero;
       nt[e] = there ? p.dt[t * p.lddt + ce] : 0.0f;
     }
 #pragma unroll
@@ -215,10 +168,9 @@ selective_scan_kernel(const ScanArgs p) {
       for (int i = 0; i < kN; ++i) {
         if (kExact) S[i] = fmaf(expm1f(st.x * A[i]), S[i], fmaf(st.y, B[i], S[i]));
         else S[i] = fmaf(mma::exp2_fast(st.x * A[i]), S[i], st.y * B[i]);
-        if (KIND != kEnds) y = fmaf(S[i], C[i], y);
+        y = fmaf(S[i], C[i], y);
       }
       share[t] = y;
-      if (KIND == kEnds) sum += st.x;
     };
     if (n_rows == kScanRows) {                                          // (the same for the whole block; no branch a row, so
 #pragma unroll                                                          // that the rows' loads and exponentials overlap)
@@ -229,10 +181,6 @@ selective_scan_kernel(const ScanArgs p) {
         share[t] = 0.0f;
         if (t < n_rows) row(t);
       }
-    }
-    if (KIND == kEnds) {
-      __syncthreads();                                                  // (steps and bc_s are written again)
-      continue;
     }
     const int first = fold_shares<kScanRows, kParts / 2>(share, part);
     constexpr int kKept = kScanRows / kParts > 0 ? kScanRows / kParts : 1;
@@ -249,35 +197,16 @@ selective_scan_kernel(const ScanArgs p) {
     }
     // (y_s is written again only behind the next chunk's first barrier, steps and bc_s only behind this chunk's second)
   }
-  if (live && KIND == kEnds) {
-#pragma unroll
-    for (int i = 0; i < kN; ++i)
-      if (n0 + i < p.states) p.ends[blockIdx.x * record + mine + i] = S[i];
-    if (part == 0) p.sums[static_cast<long long>(blockIdx.x) * p.inner + c] = sum;
-  }
-  if (live && KIND != kEnds && before + 1 == stretches) {
+  if (live) {
 #pragma unroll
     for (int i = 0; i < kN; ++i)
       if (n0 + i < p.states) Sg[n0 + i] = S[i];
   }
 }
 
-// The most stretches that a step of ``rows`` rows can have.
-static long long stretches_at_most(long long rows, int requests) { return rows / kStretchRows + requests; }
-
 template <typename T, int kParts, int kN>
-static void launch_scan(const ScanArgs& p, int rows, int requests, cudaStream_t s) {
+static void launch_scan(const ScanArgs& p, int requests, cudaStream_t s) {
   constexpr int CH = ScanShape<kParts>::CH;
-  if constexpr (sizeof(T) == 2) {
-    if (p.ends != nullptr) {
-      const dim3 grid(static_cast<unsigned>(stretches_at_most(rows, requests)), (p.inner + CH - 1) / CH);
-      constexpr int bytes = kScanRows * (2 * kParts * kN + 3 * CH) * static_cast<int>(sizeof(float));
-      static_assert(bytes <= 48 * 1024, "no opt-in needed");
-      launch_kernel(selective_scan_kernel<T, kParts, kN, kEnds>, grid, dim3(ScanShape<kParts>::kThreads), bytes, s, p);
-      launch_kernel(selective_scan_kernel<T, kParts, kN, kStretches>, grid, dim3(ScanShape<kParts>::kThreads), bytes, s, p);
-      return;
-    }
-  }
   const dim3 grid(requests, (p.inner + CH - 1) / CH);
   const int needed = kScanRows * (2 * kParts * kN + 3 * CH) * static_cast<int>(sizeof(float));
   // the rows follow one another: with no more blocks than SMs every block asks for more than half of an SM's shared memory
@@ -286,22 +215,22 @@ static void launch_scan(const ScanArgs& p, int rows, int requests, cudaStream_t 
   const int smem = alone && needed < 116 * 1024 ? 116 * 1024 : needed;
   static int raised = 48 * 1024;                               // (per instance)
   if (smem > raised) {
-    cudaFuncSetAttribute(selective_scan_kernel<T, kParts, kN, kWhole>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaFuncSetAttribute(selective_scan_kernel<T, kParts, kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     raised = smem;
   }
-  launch_kernel(selective_scan_kernel<T, kParts, kN, kWhole>, grid, dim3(ScanShape<kParts>::kThreads), smem, s, p);
+  launch_kernel(selective_scan_kernel<T, kParts, kN>, grid, dim3(ScanShape<kParts>::kThreads), smem, s, p);
 }
 
 template <typename T>
-static int dispatch_scan(const ScanArgs& p, int rows, int requests, cudaStream_t s) {
+static int dispatch_scan(const ScanArgs& p, int requests, cudaStream_t s) {
   const int n = p.states;
-  if (n <= 4) launch_scan<T, 2, 2>(p, rows, requests, s);
-  else if (n <= 8) launch_scan<T, 4, 2>(p, rows, requests, s);
-  else if (n <= 16) launch_scan<T, 8, 2>(p, rows, requests, s);
-  else if (n <= 32) launch_scan<T, 16, 2>(p, rows, requests, s);
-  else if (n <= 64) launch_scan<T, 32, 2>(p, rows, requests, s);
-  else if (n <= 128) launch_scan<T, 32, 4>(p, rows, requests, s);
-  else if (n <= 256) launch_scan<T, 32, 8>(p, rows, requests, s);
+  if (n <= 4) launch_scan<T, 2, 2>(p, requests, s);
+  else if (n <= 8) launch_scan<T, 4, 2>(p, requests, s);
+  else if (n <= 16) launch_scan<T, 8, 2>(p, requests, s);
+  else if (n <= 32) launch_scan<T, 16, 2>(p, requests, s);
+  else if (n <= 64) launch_scan<T, 32, 2>(p, requests, s);
+  else if (n <= 128) launch_scan<T, 32, 4>(p, requests, s);
+  else if (n <= 256) launch_scan<T, 32, 8>(p, requests, s);
   else return PIH_ERR_UNSUPPORTED;
   PIH_LAUNCH_CHECK();
   return 0;
@@ -311,18 +240,12 @@ static int dispatch_scan(const ScanArgs& p, int rows, int requests, cudaStream_t
 
 using namespace pih;
 
-// fp32 numbers of scratch with which a step of ``rows`` rows goes by stretches.
-extern "C" long long pih_selective_scan_scratch(int rows, int requests, int inner, int states) {
-  return stretches_at_most(rows, requests) * inner * (states + 1) + static_cast<long long>(requests) * inner * states;
-}
-
-// u, bc, z, out of ``dtype``, everything else fp32 (see ScanArgs).  ``state`` at most 256.  scratch: null, or (bf16)
-// pih_selective_scan_scratch numbers: requests of more than 256 rows go by stretches side by side.
+// u, bc, z, out of ``dtype``, everything else fp32 (see ScanArgs).  ``state`` at most 256.
 extern "C" int pih_selective_scan(int dtype, const void* u, long long ldu, const void* dt, long long lddt, const void* dt_bias,
                                   const void* A, const void* bc, long long ldbc, const void* D, const void* z, long long ldz,
                                   void* out, long long ldo, float out_scale, void* state, long long state_stride,
                                   const void* cu_q, const void* state_slots, int rows, int requests, int inner, int states,
-                                  void* scratch, void* stream) {
+                                  void* stream) {
   if (rows <= 0 || requests <= 0) return 0;
   if (inner < 1 || states < 1) return PIH_ERR_BAD_ARGUMENT;
   if ((inner + 15) / 16 > 65535) return PIH_ERR_UNSUPPORTED;
@@ -339,16 +262,8 @@ extern "C" int pih_selective_scan(int dtype, const void* u, long long ldu, const
   p.cu_q = static_cast<const int*>(cu_q);
   p.state_slots = static_cast<const int*>(state_slots);
   p.inner = inner, p.states = states;
-  p.requests = requests;
-  if (scratch != nullptr && dtype != PIH_BF16) return PIH_ERR_BAD_ARGUMENT;
-  p.ends = static_cast<float*>(scratch);
-  p.sums = p.starts = nullptr;
-  if (scratch != nullptr) {
-    p.sums = p.ends + stretches_at_most(rows, requests) * inner * states;
-    p.starts = p.sums + stretches_at_most(rows, requests) * inner;
-  }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (dtype == PIH_F32) return dispatch_scan<float>(p, rows, requests, s);
-  if (dtype == PIH_BF16) return dispatch_scan<__nv_bfloat16>(p, rows, requests, s);
+  if (dtype == PIH_F32) return dispatch_scan<float>(p, requests, s);
+  if (dtype == PIH_BF16) return dispatch_scan<__nv_bfloat16>(p, requests, s);
   return PIH_ERR_BAD_ARGUMENT;
 }

@@ -121,7 +121,6 @@ class CudaOps:
         lib.pih_linear_memory_scratch.restype = c_ll
         lib.pih_retention_chunk_scratch.restype = c_ll
         lib.pih_delta_chunk_scratch.restype = c_ll
-        lib.pih_selective_scan_scratch.restype = c_ll
 
     def _native_supports(self, block) -> bool:
         from .native_block import NativeBlocks
@@ -920,19 +919,13 @@ class CudaOps:
         if out is None:
             out = torch.empty(T, inner, dtype=u.dtype, device=u.device)
         assert out.dtype == u.dtype and out.shape == (T, inner) and out.stride(1) == 1
-        scratch = None
-        if u.dtype == torch.bfloat16 and self.chunked_memory and hasattr(step, "host_cu_q") and self._row_plan(step)[0] > self.scan_stretch_min_rows:
-            scratch = torch.empty(int(self.lib.pih_selective_scan_scratch(T, step.num_requests, inner, n)), dtype=torch.float32, device=u.device)
-            self.launches += 1
         rc = self.lib.pih_selective_scan(_DT[u.dtype], _ptr(u), c_ll(u.stride(0)), _ptr(dt), c_ll(dt.stride(0)), _ptr(dt_bias),
                                          _ptr(A), _ptr(bc), c_ll(bc.stride(0)), _ptr(D), _ptr(z), c_ll(z.stride(0)), _ptr(out),
                                          c_ll(out.stride(0)), c_float(scale), _ptr(state), c_ll(state.stride(0)),
                                          _ptr(step.cu_q), _ptr(step.state_slots), T, step.num_requests, inner, n,
-                                         _ptr(scratch), self._stream())
+                                         self._stream())
         self._check(rc, "selective_scan")
         return out
-
-    scan_stretch_min_rows = 512            # bf16 selective scans: a step whose largest request has more rows goes by stretches
 
     def rglru_scan(self, u: torch.Tensor, gates: torch.Tensor, y_pre: torch.Tensor, *, y_bias, r_bias, i_bias, lam,
                    decay_scale: float, state: torch.Tensor, step, blocks: int) -> torch.Tensor:

@@ -22,7 +22,6 @@
 // come from projections and convolutions have the storage type T.  A request's result depends on its own rows and
 // state alone, in an order of operations fixed by the row: cutting a prompt or batching it changes no bit.
 #include "common.cuh"
-#include "delta_chunks.cuh"
 
 namespace pih {
 
@@ -480,7 +479,7 @@ __global__ void delta_recurrence_kernel(const float* __restrict__ qn, const floa
                                         long long ldv, const float* __restrict__ decay, const float* __restrict__ beta,
                                         float* __restrict__ out, float* __restrict__ state, long long state_stride,
                                         const int* __restrict__ cu_q, const int* __restrict__ state_slots, int heads,
-                                        int kv_heads, int dim, int vdim, int small_rows) {
+                                        int kv_heads, int dim, int vdim) {
   extern __shared__ float smem[];
   wait_for_prior_kernels();
   launch_dependents();
@@ -489,7 +488,7 @@ __global__ void delta_recurrence_kernel(const float* __restrict__ qn, const floa
   const int j = threadIdx.x, col = blockIdx.z * cols + j;
   const int lo = cu_q[r], hi = cu_q[r + 1];
   const int slot = state_slots[r];
-  if (hi <= lo || slot < 0 || hi - lo > small_rows) return;
+  if (hi <= lo || slot < 0) return;
   const int kh = h / (heads / kv_heads);
   float* S = smem;                          // [dim][cols]
   constexpr int kVecs = kChannel ? 3 : 2;
@@ -607,7 +606,7 @@ delta_recurrence_reg_kernel(const float* __restrict__ qn, const float* __restric
                             const T* __restrict__ v, long long ldv, const float* __restrict__ decay,
                             const float* __restrict__ beta, float* __restrict__ out, float* __restrict__ state,
                             long long state_stride, const int* __restrict__ cu_q, const int* __restrict__ state_slots,
-                            int heads, int kv_heads, int vdim, int small_rows) {
+                            int heads, int kv_heads, int vdim) {
   typedef DeltaShape<kDim, kChannel> Shape;
   constexpr int kParts = Shape::kParts, kThreads = Shape::kThreads, kRows = Shape::kRows;
   constexpr int kChunk = Shape::kChunk, kCols = Shape::kCols, kPairs = kRows / 2, kTail = Shape::kTail;
@@ -620,7 +619,7 @@ delta_recurrence_reg_kernel(const float* __restrict__ qn, const float* __restric
   const int tid = threadIdx.x, part = tid % kParts, cl = tid / kParts, col0 = blockIdx.z * kCols, col = col0 + cl;
   const int lo = cu_q[r], hi = cu_q[r + 1];
   const int slot = state_slots[r];
-  if (hi <= lo || slot < 0 || hi - lo > small_rows) return;
+  if (hi <= lo || slot < 0) return;
   const int kh = h / (heads / kv_heads);
   const bool live = col < vdim;
   float* Sg = state + slot * state_stride + static_cast<long long>(h) * kDim * vdim + col;
@@ -1047,7 +1046,7 @@ extern "C" int pih_causal_conv(int dtype, const void* x, long long ldx, const vo
 template <typename T, int D, bool CH>
 static void launch_delta_reg(cudaStream_t s, const float* qn, const float* kn, const float* qk_dot, const T* v, long long ld, const float* decay,
                              const float* beta, float* out, float* state, long long state_stride, const int* cu_q,
-                             const int* state_slots, int requests, int heads, int kv_heads, int vdim, int small_rows) {
+                             const int* state_slots, int requests, int heads, int kv_heads, int vdim) {
   typedef DeltaShape<D, CH> Shape;
   const size_t needed = 2 * static_cast<size_t>(Shape::kChunk) * Shape::words(sizeof(T)) * sizeof(float);
   const dim3 grid(requests, heads, (vdim + Shape::kCols - 1) / Shape::kCols);
@@ -1062,19 +1061,19 @@ static void launch_delta_reg(cudaStream_t s, const float* qn, const float* kn, c
     raised = staged;
   }
   launch_kernel(delta_recurrence_reg_kernel<T, D, CH>, grid,
-                dim3(Shape::kThreads), staged, s, qn, kn, qk_dot, v, ld, decay, beta, out, state, state_stride, cu_q, state_slots, heads, kv_heads, vdim, small_rows);
+                dim3(Shape::kThreads), staged, s, qn, kn, qk_dot, v, ld, decay, beta, out, state, state_stride, cu_q, state_slots, heads, kv_heads, vdim);
 }
 
 template <typename T, bool CH>
 static int launch_delta(cudaStream_t s, const float* qn, const float* kn, const float* qk_dot, const T* v, long long ld, const float* decay,
                         const float* beta, float* out, float* state, long long state_stride, const int* cu_q,
-                        const int* state_slots, int requests, int heads, int kv_heads, int dim, int vdim, int small_rows) {
+                        const int* state_slots, int requests, int heads, int kv_heads, int dim, int vdim) {
   const bool words = sizeof(T) == 4 || (ld % 2 == 0 && vdim % 2 == 0 && (reinterpret_cast<uintptr_t>(v) & 3) == 0);
   switch (words ? dim : 0) {                                   // (values are copied in 32-bit words)
 #define PIH_DELTA_REG(D)                                                                                               \
   case D:                                                                                                              \
     launch_delta_reg<T, D, CH>(s, qn, kn, qk_dot, v, ld, decay, beta, out, state, state_stride, cu_q, state_slots, requests,   \
-                               heads, kv_heads, vdim, small_rows);                                                                 \
+                               heads, kv_heads, vdim);                                                                 \
     break
     PIH_DELTA_REG(16);
     PIH_DELTA_REG(32);
@@ -1092,32 +1091,20 @@ static int launch_delta(cudaStream_t s, const float* qn, const float* kn, const 
                              static_cast<int>(smem));
       const dim3 grid(requests, heads, (vdim + cols - 1) / cols);
       launch_kernel(delta_recurrence_kernel<T, CH>, grid, dim3(cols), smem, s, qn, kn, v, ld, decay, beta, out, state,
-                    state_stride, cu_q, state_slots, heads, kv_heads, dim, vdim, small_rows);
+                    state_stride, cu_q, state_slots, heads, kv_heads, dim, vdim);
     }
   }
   PIH_LAUNCH_CHECK();
   return 0;
 }
 
-// fp32 numbers of chunk scratch that a step of ``rows`` rows needs; 0: its sizes do not go by chunks.
-extern "C" long long pih_delta_chunk_scratch(int dtype, int rows, int requests, int heads, int dim, int vdim) {
-  return dtype == PIH_BF16 && delta_takes_chunks(heads, dim, vdim) ? delta_chunk_scratch(rows, requests, heads, dim, vdim) : 0;
-}
-
-// chunk_scratch: null, or pih_delta_chunk_scratch numbers, 16-byte aligned: requests of more than 16 rows go by chunks;
-// ``small`` 0 then says that there are no others.
 extern "C" int pih_gated_delta_rule(int dtype, const void* qkv, long long ld, const void* b, long long ldb, int a_dtype,
                                     const void* a, long long lda, int channels, const void* decay_log,
                                     const void* decay_bias, void* scratch, void* out, void* state, long long state_stride,
                                     const void* cu_q, const void* state_slots, int rows, int requests, int heads,
-                                    int kv_heads, int dim, int vdim, float unit_eps, float q_scale, void* chunk_scratch,
-                                    int small, void* stream) {
+                                    int kv_heads, int dim, int vdim, float unit_eps, float q_scale, void* stream) {
   if (rows <= 0 || requests <= 0) return 0;
   if (heads % kv_heads) return PIH_ERR_BAD_ARGUMENT;
-  if (chunk_scratch != nullptr && (dtype != PIH_BF16 || !delta_takes_chunks(heads, dim, vdim) ||
-                                   reinterpret_cast<uintptr_t>(scratch) % 16 || reinterpret_cast<uintptr_t>(chunk_scratch) % 16))
-    return PIH_ERR_UNSUPPORTED;
-  const int small_rows = chunk_scratch != nullptr ? kDeltaSmallRows : 0x7fffffff;
   if (heads > 65535 || (vdim + 15) / 16 > 65535) return PIH_ERR_UNSUPPORTED;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const long long qk_size = static_cast<long long>(kv_heads) * dim;
@@ -1140,16 +1127,10 @@ extern "C" int pih_gated_delta_rule(int dtype, const void* qkv, long long ld, co
     float* st = static_cast<float*>(state);                                                                            \
     const int* cu = static_cast<const int*>(cu_q);                                                                     \
     const int* slots = static_cast<const int*>(state_slots);                                                           \
-    if (chunk_scratch != nullptr) {                                                                                    \
-      const DeltaChunkArgs p = {qn, kn, qk_dot, decay, beta, static_cast<const bf16*>(static_cast<const void*>(v)), ld, o, st, \
-                                state_stride, static_cast<float*>(chunk_scratch), cu, slots, requests, heads, kv_heads, vdim}; \
-      const int rc = launch_delta_chunks(s, p, dim, channels != 0, rows);                                              \
-      if (rc != 0 || !small) return rc;                                                                                \
-    }                                                                                                                  \
     return channels ? launch_delta<T, true>(s, qn, kn, qk_dot, v, ld, decay, beta, o, st, state_stride, cu, slots, requests,   \
-                                            heads, kv_heads, dim, vdim, small_rows)                                                \
+                                            heads, kv_heads, dim, vdim)                                                \
                     : launch_delta<T, false>(s, qn, kn, qk_dot, v, ld, decay, beta, o, st, state_stride, cu, slots, requests,  \
-                                             heads, kv_heads, dim, vdim, small_rows);                                  \
+                                             heads, kv_heads, dim, vdim);                                              \
   } while (0)
   if (dtype == PIH_F32 && a_dtype == PIH_F32) PIH_DELTA(float, float);
   if (dtype == PIH_BF16 && a_dtype == PIH_BF16) PIH_DELTA(bf16, bf16);

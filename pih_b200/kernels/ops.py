@@ -120,7 +120,6 @@ class CudaOps:
         lib.pih_moe_route_words.restype = c_ll
         lib.pih_linear_memory_scratch.restype = c_ll
         lib.pih_retention_chunk_scratch.restype = c_ll
-        lib.pih_delta_chunk_scratch.restype = c_ll
 
     def _native_supports(self, block) -> bool:
         from .native_block import NativeBlocks
@@ -771,16 +770,14 @@ class CudaOps:
         assert beta.shape[1] >= heads and decay.shape[1] >= per_row and decay_bias.numel() == per_row
         scratch = torch.empty(T * (2 * kv_heads * key_dim + kv_heads + heads + per_row), dtype=torch.float32, device=qkv.device)
         out = torch.empty(T, heads, value_dim, dtype=torch.float32, device=qkv.device)
-        chunk_scratch, small = self._chunk_scratch(qkv.dtype, step, lambda: self.lib.pih_delta_chunk_scratch(
-            _DT[qkv.dtype], T, step.num_requests, heads, key_dim, value_dim), qkv.device)
         rc = self.lib.pih_gated_delta_rule(_DT[qkv.dtype], _ptr(qkv), c_ll(qkv.stride(0)), _ptr(beta), c_ll(beta.stride(0)),
                                            _DT[decay.dtype], _ptr(decay), c_ll(decay.stride(0)), 1 if channels else 0,
                                            _ptr(decay_log), _ptr(decay_bias), _ptr(scratch), _ptr(out), _ptr(state),
                                            c_ll(state.stride(0)), _ptr(step.cu_q), _ptr(step.state_slots), T,
                                            step.num_requests, heads, kv_heads, key_dim, value_dim, c_float(unit_eps),
-                                           c_float(q_scale), _ptr(chunk_scratch), small, self._stream())
+                                           c_float(q_scale), self._stream())
         self._check(rc, "gated_delta_rule")
-        self.launches += 1 + (2 + small if chunk_scratch is not None else 0)      # (of two to five kernels)
+        self.launches += 1                                     # two kernels
         return out
 
     def gated_rmsnorm(self, o: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor, eps: float, activation: str = "silu",

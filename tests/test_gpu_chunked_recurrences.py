@@ -1,5 +1,6 @@
-"""Recurrences that take a prompt chunk by chunk, against their definition in float64 — remainders of a chunk, requests that go
-token by token and requests of padding beside them, a state carried in — and against the token loop's own error."""
+"""Recurrences of prompts: chunk by chunk against the definition in float64 — remainders of a chunk, requests that go token by
+token and requests of padding beside them, a state carried in — and against the token loop's own error; token by token, bits
+that are the request's own."""
 import pytest
 import torch
 
@@ -66,51 +67,71 @@ def test_retention(dim, vdim, lens):
         assert torch.equal(state[0], first[0]) and torch.equal(state[len(lens) + 1:], first[len(lens) + 1:])
 
 
-@pytest.mark.parametrize("channels", [True, False])
-@pytest.mark.parametrize("dim, vdim", [(64, 64), (128, 128), (64, 192)])
-@pytest.mark.parametrize("lens", [[65], [64, 128], [130, 1, 17, 16, 200], [700]])
-@pytest.mark.parametrize("pace", [0.02, 1.0, 30.0])          # decays next to one, ordinary ones, channels that forget at once
-def test_delta_rule(dim, vdim, lens, channels, pace):
-    ops, heads, kv_heads = _ops(), 4, 2
-    step, places = _requests(lens)
+def _delta(ops, T, lens, slots, qkv, beta, a, bias, log, state, dim, vdim, heads, kv_heads):
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    step = _step(list(range(T)), [0] * T, cu, slots)
+    return ops.gated_delta_rule(qkv, beta, a, decay_log=log, decay_bias=bias, state=state, step=step, heads=heads,
+                                kv_heads=kv_heads, key_dim=dim, value_dim=vdim, unit_eps=1e-6, q_scale=dim ** -0.5)
+
+
+@pytest.mark.parametrize("dim, vdim", [(64, 64), (128, 128)])
+@pytest.mark.parametrize("cut", [1, 64, 300])
+def test_delta_rule_by_the_request(dim, vdim, cut):
+    """A request's bits are its own: alone, cut in two, beside longer and shorter ones.  A decay of zero erases the state, one
+    that is no number reaches every row from its own on and none before."""
+    ops, heads, kv_heads, lens = _ops(), 4, 2, [40, 700, 1, 130]
     T, QK = sum(lens), kv_heads * dim
-    g = torch.Generator().manual_seed(dim + T)
+    g = torch.Generator().manual_seed(dim + cut)
     qkv = (torch.randn(T, 2 * QK + heads * vdim, generator=g) * 0.7).bfloat16().to(DEV)
     beta = torch.randn(T, heads, generator=g).bfloat16().to(DEV)
-    per = dim if channels else 1
-    a, bias = torch.randn(T, heads * per, generator=g).to(DEV), (torch.randn(heads * per, generator=g) * 0.5).to(DEV)
-    log = torch.log(torch.tensor([0.2, 1.0, 2.0, 0.5])).to(DEV) + torch.log(torch.tensor(pace)).to(DEV)
-    first = torch.randn(len(lens) + 2, heads * dim * vdim + 4, generator=g).to(DEV)
-    results = []
-    for chunked in (True, False):
-        state, ops.chunk_min_rows = first.clone(), 64 if chunked else 1 << 30
-        o = ops.gated_delta_rule(qkv, beta, a, decay_log=log, decay_bias=bias, state=state, step=step, heads=heads,
-                                 kv_heads=kv_heads, key_dim=dim, value_dim=vdim, unit_eps=1e-6, q_scale=dim ** -0.5)
-        results.append((o, state))
-    ops.chunk_min_rows = type(ops).chunk_min_rows
-    ops.check_errors()
-    x = qkv.double()
-    unit = lambda t: t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6)                     # noqa: E731
-    q, k = (unit(t.view(T, kv_heads, dim)).repeat_interleave(heads // kv_heads, 1) for t in (x[:, :QK], x[:, QK:2 * QK]))
-    q, v = q * dim ** -0.5, x[:, 2 * QK:].view(T, heads, vdim)
-    z = (a.double() + bias.double()).view(T, heads, per)
-    decay = torch.exp(-torch.exp(log.double())[:, None] * torch.nn.functional.softplus(z)).expand(T, heads, dim)
-    write = torch.sigmoid(beta.double())
-    errors = [0.0, 0.0]
-    for lo, hi, slot in places:
-        S = first[slot, :-4].double().view(heads, dim, vdim)
-        ref = torch.empty(hi - lo, heads, vdim, dtype=F64, device=DEV)
-        for t in range(lo, hi):
-            S = decay[t, :, :, None] * S
-            u = write[t, :, None] * (v[t] - (k[t, :, None] @ S)[:, 0])
-            S = S + k[t, :, :, None] * u[:, None]
-            ref[t - lo] = (q[t, :, None] @ S)[:, 0]
-        for i, (o, state) in enumerate(results):
-            errors[i] = max(errors[i], float((o[lo:hi].double() - ref).norm() / ref.norm()),
-                            float((state[slot, :-4].double().view_as(S) - S).norm() / S.norm()))
-    print("chunks", errors[0], "tokens", errors[1])
-    # 32-bit sums of chains of up to 128 + 64 terms, where the token loop adds 4 and then by halves: a few times 2^-24 either way
-    assert errors[0] < 8 * 2.0 ** -24 and errors[0] < 3 * errors[1]
-    for _, state in results:
-        assert torch.equal(state[0], first[0]) and torch.equal(state[len(lens) + 1:], first[len(lens) + 1:])
-        assert torch.equal(state[:, -4:], first[:, -4:])
+    a, bias = torch.randn(T, heads * dim, generator=g).to(DEV), torch.zeros(heads * dim, device=DEV)
+    log = torch.zeros(heads, device=DEV)
+    first = torch.randn(4, heads * dim * vdim, generator=g).to(DEV)
+    rest = (bias, log)
+    state = first.clone()
+    together = _delta(ops, T, lens, [0, 1, 2, 3], qkv, beta, a, *rest, state, dim, vdim, heads, kv_heads)
+    alone = first.clone()
+    lo, hi = 40, 740
+    for x, y in ((lo, lo + cut), (lo + cut, hi)):
+        o = _delta(ops, y - x, [y - x], [1], qkv[x:y], beta[x:y], a[x:y], *rest, alone, dim, vdim, heads, kv_heads)
+        assert torch.equal(o, together[x:y])
+    assert torch.equal(alone[1], state[1]) and torch.equal(alone[0], first[0])
+    # softplus(inf) = inf: every channel's decay is zero, the row sees only what it writes itself
+    wiped = a.clone()
+    wiped[lo + 200] = float("inf")
+    state2, other = first.clone(), first.clone()
+    other[1] = 1e30
+    o1 = _delta(ops, T, lens, [0, 1, 2, 3], qkv, beta, wiped, *rest, state2, dim, vdim, heads, kv_heads)
+    x = slice(lo + 200, hi)
+    o2 = _delta(ops, 500, [500], [1], qkv[x], beta[x], wiped[x], *rest, other, dim, vdim, heads, kv_heads)
+    assert torch.equal(o1[x], o2) and torch.equal(other[1], state2[1]) and torch.equal(o1[lo:lo + 200], together[lo:lo + 200])
+    spoilt = a.clone()
+    spoilt[lo + 203, :dim] = float("nan")                                       # the first head's
+    state3 = first.clone()
+    o3 = _delta(ops, T, lens, [0, 1, 2, 3], qkv, beta, spoilt, *rest, state3, dim, vdim, heads, kv_heads)
+    assert torch.equal(o3[:lo + 203], together[:lo + 203]) and bool(o3[lo + 203:hi, 0].isnan().all())
+    assert bool(state3[1].view(heads, -1)[0].isnan().all()) and torch.equal(o3[hi:], together[hi:])
+
+
+@pytest.mark.parametrize("cut", [1, 16, 256, 511])
+def test_selective_scan_by_the_request(cut):
+    """The same of the selective scan: alone, cut in two, beside others."""
+    ops, inner, n, lens = _ops(), 40, 16, [300, 1100, 1, 513]
+    T = sum(lens)
+    g = torch.Generator().manual_seed(cut)
+    u, z = (torch.randn(T, inner, generator=g).bfloat16().to(DEV) for _ in range(2))
+    bc = torch.randn(T, 2 * n, generator=g).bfloat16().to(DEV)
+    dt, bias, D = (torch.randn(*s, generator=g).to(DEV) for s in ((T, inner), (inner,), (inner,)))
+    A = -torch.exp(torch.randn(inner, n, generator=g) * 2 - 3).to(DEV)
+    first = torch.randn(4, inner * n, generator=g).to(DEV)
+
+    def scan(x, y, cu, slots, state):
+        step = _step(list(range(y - x)), [0] * (y - x), cu, slots)
+        return ops.selective_scan(u[x:y], dt[x:y], bc[x:y], z[x:y], dt_bias=bias, A=A, D=D, state=state, step=step)
+    state, alone = first.clone(), first.clone()
+    together = scan(0, T, [0, 300, 1400, 1401, T], [0, 1, 2, 3], state)
+    for x, y in ((300, 300 + cut), (300 + cut, 1400)):
+        assert torch.equal(scan(x, y, [0, y - x], [1], alone), together[x:y])
+    assert torch.equal(alone[1], state[1]) and torch.equal(alone[0], first[0])

@@ -1,4 +1,4 @@
-// Chunks of 64 rows of the requests of a step, for recurrences that take a long request's rows chunk by chunk.
+// Chunks of 64 rows of the requests of a step, for a recurrence that takes a long request's rows chunk by chunk.
 #pragma once
 
 #include "common.cuh"
@@ -8,13 +8,13 @@ namespace chunks {
 
 constexpr int kRows = 64;
 
-struct Place { int request, first, rows, index; };           // rows first .. first + rows - 1 of the step; index: of the step
+struct Place { int request, first, rows; };                  // rows first .. first + rows - 1 of the step
 
 // The x-th chunk of the step's requests that have more than small_rows rows (request -1: there is none); for every thread
 // of the block.
 __device__ __forceinline__ Place find(const int* cu_q, const int* state_slots, int requests, int small_rows, int x, Place* shared) {
   if (threadIdx.x == 0) {
-    Place c = {-1, 0, 0, x};
+    Place c = {-1, 0, 0};
     int t = x;
     for (int r = 0; r < requests; ++r) {
       const int lo = cu_q[r], n = cu_q[r + 1] - lo;

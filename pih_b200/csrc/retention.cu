@@ -5,16 +5,18 @@
 //   retention_recurrence   per token  S <- S + (decay - 1) S + k v^T,  o = S^T q,  from the request's state slot; S in
 //                          shared memory (any key size), or in registers for the key sizes that have an instance
 //
-// The order of the additions of a read-out is fixed by the kernel: it does not depend on how a sequence is cut into
-// steps or on what else a step holds.
+// The order of the additions of a read-out is fixed by the kernel and by what its request brings to the step: it does not
+// depend on what else the step holds, and with the token loop (32-bit, and bf16 requests of up to ``small_rows`` rows)
+// not on how a sequence is cut into steps either.
 //
-// bf16, a step with a request of more than 64 rows: requests of more than 16 rows go by chunks of 64 rows instead, all
-// chunks side by side, in 32-bit products on the CUDA cores (the same precision; the token loop is a chain of 0.27 us a
-// token on 32 of the 148 SMs, 560 us for 2048 rows of 8 heads of 128 x 128):
+// bf16 requests of more than ``small_rows`` rows go by chunks of 64 rows instead, all chunks side by side, in 32-bit
+// products on the CUDA cores (closer to the exact sums than the token loop, which is a chain of 0.27 us a token on 32 of
+// the 148 SMs for 8 heads of 128 x 128):
 //   retention_chunk_state   U = sum_j decay^(end - j) k_j v_j^T, what a chunk adds to the state
 //   retention_state_pass    the chunks in order: the state in front of each takes U's place; S <- decay^rows S + U
 //   retention_chunk_out     o_i = decay^(i + 1) S^T q_i + sum_{j <= i} decay^(i - j) (q_i . k_j) v_j
-// decay^n is formed as exp(n log1p(decay - 1)).
+// decay^n is formed as exp(n log1p(decay - 1)).  Steps whose chunks do not fit the scratch go in waves of as many as do, the
+// state in the slot in between.
 #include "chunks.cuh"
 #include "common.cuh"
 
@@ -227,8 +229,6 @@ retention_recurrence_reg_kernel(const float* __restrict__ qf, const float* __res
 }
 
 // ---- by chunks ----------------------------------------------------------------------------------------------------------
-constexpr int kRetentionSmallRows = 16;                    // requests of at most this many rows go token by token
-
 struct RetentionArgs {
   const float* q;                                          // rotated, [rows, heads, dim]
   const float* k;                                          // rotated and scaled
@@ -238,10 +238,11 @@ struct RetentionArgs {
   float* out;
   float* state;
   long long state_stride;
-  float* chunk_states;                                     // [chunks, heads, dim, vdim]
+  float* chunk_states;                                     // of the wave: [chunks, heads, dim, vdim]
   const int* cu_q;
   const int* state_slots;
-  int requests, heads, vdim;
+  int requests, heads, vdim, small_rows;
+  int from, chunks;                                        // the wave: its first chunk of the step's, how many
 };
 
 __device__ __forceinline__ float decay_power(float log_decay, int n) { return n == 0 ? 1.0f : expf(log_decay * static_cast<float>(n)); }
@@ -258,7 +259,7 @@ retention_chunk_state_kernel(const RetentionArgs p) {
   __shared__ float power[chunks::kRows];
   wait_for_prior_kernels();
   launch_dependents();
-  const chunks::Place c = chunks::find(p.cu_q, p.state_slots, p.requests, kRetentionSmallRows, blockIdx.x, &place);
+  const chunks::Place c = chunks::find(p.cu_q, p.state_slots, p.requests, p.small_rows, p.from + blockIdx.x, &place);
   if (c.request < 0) return;
   const int h = blockIdx.y, v0 = blockIdx.z * VT, tid = threadIdx.x;
   chunks::load_rows<DIM, DIM>(ks, p.k + (static_cast<long long>(c.first) * p.heads + h) * DIM, static_cast<long long>(p.heads) * DIM, c.rows);
@@ -274,7 +275,7 @@ retention_chunk_state_kernel(const RetentionArgs p) {
   chunks::clear(U);
   chunks::multiply_outer<RM, RN>(U, ks, DIM, vs, VT, (c.rows + 3) & ~3);
   const int tx = tid & 15, ty = tid >> 4;
-  float* to = p.chunk_states + ((static_cast<long long>(c.index) * p.heads + h) * DIM + ty * RM) * p.vdim + v0 + 4 * tx;
+  float* to = p.chunk_states + ((static_cast<long long>(blockIdx.x) * p.heads + h) * DIM + ty * RM) * p.vdim + v0 + 4 * tx;
 #pragma unroll
   for (int i = 0; i < RM; ++i)
 #pragma unroll
@@ -283,7 +284,7 @@ retention_chunk_state_kernel(const RetentionArgs p) {
           make_float4(U[i][2 * g].x, U[i][2 * g].y, U[i][2 * g + 1].x, U[i][2 * g + 1].y);
 }
 
-// Block (request, head, 128 pieces of four numbers of S): a stream over the chunks, eight of them asked for ahead.
+// Block (request, head, 128 pieces of four numbers of S): a stream over the wave's chunks, eight of them asked for ahead.
 __global__ void __launch_bounds__(128)
 retention_state_pass_kernel(const RetentionArgs p, int dim) {
   __shared__ int first;
@@ -291,30 +292,31 @@ retention_state_pass_kernel(const RetentionArgs p, int dim) {
   launch_dependents();
   const int r = blockIdx.x, h = blockIdx.y;
   const int n = p.cu_q[r + 1] - p.cu_q[r], slot = p.state_slots[r];
-  if (n <= kRetentionSmallRows || slot < 0) return;
-  if (threadIdx.x == 0) first = chunks::first_of(p.cu_q, p.state_slots, kRetentionSmallRows, r);
+  if (n <= p.small_rows || slot < 0) return;
+  if (threadIdx.x == 0) first = chunks::first_of(p.cu_q, p.state_slots, p.small_rows, r);
   __syncthreads();
+  const int count = (n + chunks::kRows - 1) / chunks::kRows;
+  const int lo = max(0, p.from - first), hi = min(count, p.from + p.chunks - first);     // the request's chunks of this wave
   const long long matrix = static_cast<long long>(dim) * p.vdim, at = (static_cast<long long>(blockIdx.z) * 128 + threadIdx.x) * 4;
-  if (at >= matrix) return;
+  if (lo >= hi || at >= matrix) return;
   float* Sg = p.state + slot * p.state_stride + h * matrix + at;
   float4 S = make_float4(Sg[0], Sg[1], Sg[2], Sg[3]);
-  float* U = p.chunk_states + (static_cast<long long>(first) * p.heads + h) * matrix + at;
   const long long step = p.heads * matrix;
-  const int count = (n + chunks::kRows - 1) / chunks::kRows;
+  float* U = p.chunk_states + (static_cast<long long>(first + lo - p.from) * p.heads + h) * matrix + at;
   const float lg = log1pf(p.decay_m1[h]), whole = decay_power(lg, chunks::kRows);
   constexpr int kAhead = 8;
   float4 u[kAhead];
 #pragma unroll
   for (int i = 0; i < kAhead; ++i)
-    if (i < count) u[i] = *reinterpret_cast<const float4*>(U + i * step);
-  for (int c0 = 0; c0 < count; c0 += kAhead) {
+    if (lo + i < hi) u[i] = *reinterpret_cast<const float4*>(U + i * step);
+  for (int c0 = lo; c0 < hi; c0 += kAhead) {
 #pragma unroll
     for (int i = 0; i < kAhead; ++i) {
       const int c = c0 + i;
-      if (c >= count) break;
+      if (c >= hi) break;
       const float4 add = u[i];
-      if (c + kAhead < count) u[i] = *reinterpret_cast<const float4*>(U + (c + kAhead) * step);
-      *reinterpret_cast<float4*>(U + c * step) = S;
+      if (c + kAhead < hi) u[i] = *reinterpret_cast<const float4*>(U + (c + kAhead - lo) * step);
+      *reinterpret_cast<float4*>(U + (c - lo) * step) = S;
       const float f = c + 1 < count ? whole : decay_power(lg, n - c * chunks::kRows);
       S.x = fmaf(f, S.x, add.x);
       S.y = fmaf(f, S.y, add.y);
@@ -343,7 +345,7 @@ retention_chunk_out_kernel(const RetentionArgs p) {
   __shared__ float power[chunks::kRows + 1];
   wait_for_prior_kernels();
   launch_dependents();
-  const chunks::Place c = chunks::find(p.cu_q, p.state_slots, p.requests, kRetentionSmallRows, blockIdx.x, &place);
+  const chunks::Place c = chunks::find(p.cu_q, p.state_slots, p.requests, p.small_rows, p.from + blockIdx.x, &place);
   if (c.request < 0) return;
   const int h = blockIdx.y, v0 = blockIdx.z * VT, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const long long at = (static_cast<long long>(c.first) * p.heads + h) * DIM, ld = static_cast<long long>(p.heads) * DIM;
@@ -368,7 +370,7 @@ retention_chunk_out_kernel(const RetentionArgs p) {
   constexpr int RN = VT / 16;
   float2 o[4][RN / 2];
   chunks::clear(o);
-  const float* state = p.chunk_states + (static_cast<long long>(c.index) * p.heads + h) * DIM * p.vdim + v0;
+  const float* state = p.chunk_states + (static_cast<long long>(blockIdx.x) * p.heads + h) * DIM * p.vdim + v0;
 #pragma unroll 1
   for (int d0 = 0; d0 < DIM; d0 += chunks::kRows) {
     __syncthreads();                                       // (what lay there is done with)
@@ -411,25 +413,33 @@ static bool retention_takes_chunks(int dtype, const void* v, long long ldv, int 
          reinterpret_cast<uintptr_t>(v) % 16 == 0 && ldv % 8 == 0;
 }
 
-// fp32 numbers of chunk scratch that a step of ``rows`` rows needs; 0: its sizes do not go by chunks.
+// fp32 numbers of chunk scratch for a step of ``rows`` rows whose requests of more than ``small_rows`` rows go by chunks, at most
+// ``most`` of them (or one chunk's); 0: its sizes do not go by chunks.
 extern "C" long long pih_retention_chunk_scratch(int dtype, const void* v, long long ldv, int rows, int requests, int heads, int dim,
-                                                 int vdim) {
+                                                 int vdim, int small_rows, long long most) {
   if (!retention_takes_chunks(dtype, v, ldv, heads, dim, vdim)) return 0;
-  return chunks::at_most(rows, requests, kRetentionSmallRows) * heads * dim * vdim;
+  const long long each = static_cast<long long>(heads) * dim * vdim, fit = most / each > 1 ? most / each : 1;
+  const long long chunks = chunks::at_most(rows, requests, small_rows);
+  return (chunks < fit ? chunks : fit) * each;
 }
 
 template <int DIM, int VT>
-static int launch_retention_chunks(cudaStream_t s, const RetentionArgs& p, int rows) {
-  const unsigned count = static_cast<unsigned>(chunks::at_most(rows, p.requests, kRetentionSmallRows)), tiles = p.vdim / VT;
+static int launch_retention_chunks(cudaStream_t s, RetentionArgs p, int rows, long long scratch) {
+  const unsigned tiles = p.vdim / VT;
   constexpr size_t state_bytes = sizeof(float) * chunks::kRows * (DIM + VT), out_bytes = retention_out_bytes<DIM, VT>();
   cudaFuncSetAttribute(retention_chunk_state_kernel<DIM, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(state_bytes));
   cudaFuncSetAttribute(retention_chunk_out_kernel<DIM, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(out_bytes));
-  launch_kernel(retention_chunk_state_kernel<DIM, VT>, dim3(count, p.heads, tiles), dim3(256), state_bytes, s, p);
-  PIH_LAUNCH_CHECK();
-  launch_kernel(retention_state_pass_kernel, dim3(p.requests, p.heads, (DIM * p.vdim / 4 + 127) / 128), dim3(128), 0, s, p, DIM);
-  PIH_LAUNCH_CHECK();
-  launch_kernel(retention_chunk_out_kernel<DIM, VT>, dim3(count, p.heads, tiles), dim3(256), out_bytes, s, p);
-  PIH_LAUNCH_CHECK();
+  const long long count = chunks::at_most(rows, p.requests, p.small_rows), fit = scratch / (static_cast<long long>(p.heads) * DIM * p.vdim);
+  for (long long from = 0; from < count; from += fit) {
+    p.from = static_cast<int>(from);
+    p.chunks = static_cast<int>(count - from < fit ? count - from : fit);
+    launch_kernel(retention_chunk_state_kernel<DIM, VT>, dim3(p.chunks, p.heads, tiles), dim3(256), state_bytes, s, p);
+    PIH_LAUNCH_CHECK();
+    launch_kernel(retention_state_pass_kernel, dim3(p.requests, p.heads, (DIM * p.vdim / 4 + 127) / 128), dim3(128), 0, s, p, DIM);
+    PIH_LAUNCH_CHECK();
+    launch_kernel(retention_chunk_out_kernel<DIM, VT>, dim3(p.chunks, p.heads, tiles), dim3(256), out_bytes, s, p);
+    PIH_LAUNCH_CHECK();
+  }
   return 0;
 }
 
@@ -456,17 +466,20 @@ static void launch_retention_in_registers(cudaStream_t s, const float* qf, const
 // qk [rows, ld]: q heads then k heads ([heads, dim] each); v [rows, ldv]: [heads, vdim]; freq fp32 [rot / 2] (null: no
 // rotation); decay_m1 fp32 [heads]: decay - 1; scratch fp32 [2 * rows * heads * dim]; out fp32 [rows, heads, vdim];
 // state fp32: S of (slot, head) at state + slot * state_stride + head * dim * vdim, [dim, vdim].  chunk_scratch: null, or
-// pih_retention_chunk_scratch numbers, 16-byte aligned: requests of more than 16 rows go by chunks; ``small`` 0 then says that
-// there are no others.
+// chunk_numbers of fp32, 16-byte aligned, one chunk's or more (pih_retention_chunk_scratch): requests of more than small_rows
+// rows go by chunks.
 extern "C" int pih_retention(int dtype, const void* qk, long long ld, const void* v, long long ldv, const void* freq, int rot,
                              const void* positions, const void* decay_m1, float key_scale, void* scratch, void* out,
                              void* state, long long state_stride, const void* cu_q, const void* state_slots, int rows,
-                             int requests, int heads, int dim, int vdim, void* chunk_scratch, int small, void* stream) {
+                             int requests, int heads, int dim, int vdim, void* chunk_scratch, long long chunk_numbers, int small_rows,
+                             void* stream) {
   if (rows <= 0 || requests <= 0) return 0;
   if (chunk_scratch != nullptr && (!retention_takes_chunks(dtype, v, ldv, heads, dim, vdim) ||
                                    reinterpret_cast<uintptr_t>(chunk_scratch) % 16 || reinterpret_cast<uintptr_t>(scratch) % 16))
     return PIH_ERR_UNSUPPORTED;
-  const int small_rows = chunk_scratch != nullptr ? kRetentionSmallRows : 0x7fffffff;
+  if (chunk_scratch != nullptr && (small_rows < 0 || chunk_numbers < static_cast<long long>(heads) * dim * vdim))
+    return PIH_ERR_BAD_ARGUMENT;
+  if (chunk_scratch == nullptr) small_rows = 0x7fffffff;
   if (rot < 0 || rot > dim || (rot & 1) || (rot > 0 && freq == nullptr)) return PIH_ERR_BAD_ARGUMENT;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int cols = vdim >= 64 ? 64 : 32;
@@ -494,12 +507,12 @@ extern "C" int pih_retention(int dtype, const void* qk, long long ld, const void
       const RetentionArgs p = {qf, kf, static_cast<const bf16*>(v), ldv, static_cast<const float*>(decay_m1),          \
                                static_cast<float*>(out), static_cast<float*>(state), state_stride,                     \
                                static_cast<float*>(chunk_scratch), static_cast<const int*>(cu_q),                      \
-                               static_cast<const int*>(state_slots), requests, heads, vdim};                           \
-      const int rc = dim == 128 ? (vdim % 128 ? launch_retention_chunks<128, 64>(s, p, rows)                           \
-                                              : launch_retention_chunks<128, 128>(s, p, rows))                         \
-                                : (vdim % 128 ? launch_retention_chunks<64, 64>(s, p, rows)                            \
-                                              : launch_retention_chunks<64, 128>(s, p, rows));                         \
-      if (rc != 0 || !small) return rc;                                                                                \
+                               static_cast<const int*>(state_slots), requests, heads, vdim, small_rows, 0, 0};         \
+      const int rc = dim == 128 ? (vdim % 128 ? launch_retention_chunks<128, 64>(s, p, rows, chunk_numbers)            \
+                                              : launch_retention_chunks<128, 128>(s, p, rows, chunk_numbers))          \
+                                : (vdim % 128 ? launch_retention_chunks<64, 64>(s, p, rows, chunk_numbers)             \
+                                              : launch_retention_chunks<64, 128>(s, p, rows, chunk_numbers));          \
+      if (rc != 0) return rc;                                                                                          \
     }                                                                                                                  \
     if (in_registers) {                                                                                                \
       switch (dim) {                                                                                                   \

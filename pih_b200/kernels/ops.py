@@ -1161,29 +1161,36 @@ class CudaOps:
         scratch = torch.empty(2 * T * heads * key_dim, dtype=torch.float32, device=qk.device)
         out = torch.empty(T, heads, value_dim, dtype=torch.float32, device=qk.device)
         rot = 2 * frequencies.shape[0] if frequencies is not None else 0
-        chunk_scratch, small = self._chunk_scratch(qk.dtype, step, lambda: self.lib.pih_retention_chunk_scratch(
-            _DT[qk.dtype], _ptr(v), c_ll(v.stride(0)), T, step.num_requests, heads, key_dim, value_dim), qk.device)
+        # bf16 requests of more than ``chunk_min_rows`` rows go by chunks of 64 rows, if the step may hold one
+        chunk_scratch, numbers = None, 0
+        if qk.dtype == torch.bfloat16 and self.chunked_memory:
+            largest = self._row_plan(step)[0] if hasattr(step, "host_cu_q") else T
+            if largest > self.chunk_min_rows:
+                numbers = int(self.lib.pih_retention_chunk_scratch(
+                    _DT[qk.dtype], _ptr(v), c_ll(v.stride(0)), T, step.num_requests, heads, key_dim, value_dim,
+                    self.chunk_min_rows, c_ll(self.chunk_scratch_numbers)))
+            if numbers > 0:
+                chunk_scratch = torch.empty(numbers, dtype=torch.float32, device=qk.device)
+                self.launches += 3                             # (a wave; more where the scratch is short)
         rc = self.lib.pih_retention(_DT[qk.dtype], _ptr(qk), c_ll(qk.stride(0)), _ptr(v), c_ll(v.stride(0)), _ptr(frequencies),
                                     rot, _ptr(step.positions), _ptr(decay_minus_one), c_float(key_scale), _ptr(scratch),
                                     _ptr(out), _ptr(state), c_ll(state.stride(0)), _ptr(step.cu_q), _ptr(step.state_slots),
-                                    T, step.num_requests, heads, key_dim, value_dim, _ptr(chunk_scratch), small, self._stream())
+                                    T, step.num_requests, heads, key_dim, value_dim, _ptr(chunk_scratch), c_ll(numbers),
+                                    self.chunk_min_rows, self._stream())
         self._check(rc, "retention")
-        self.launches += 1 + (2 + small if chunk_scratch is not None else 0)      # (of two to five kernels)
+        self.launches += 1                                     # two kernels
         return out
 
-    chunk_min_rows = 64                    # bf16 recurrences: a step whose largest request has more rows goes by chunks
-
-    def _chunk_scratch(self, dtype: torch.dtype, step, need, device):
-        """(scratch of a recurrence that goes by chunks of 64 rows or None, whether the step has requests of at most 16 rows
-        beside them).  bf16 only: in 32-bit a row's bits do not depend on where a request is cut.  A step whose largest
-        request has no more than 64 rows stays with the token loop, which 64 rows take no longer than the chunks' kernels."""
-        if dtype != torch.bfloat16 or not self.chunked_memory or not hasattr(step, "host_cu_q"):
-            return None, 1
-        big, small_rows, _ = self._row_plan(step)
-        numbers = need() if big > self.chunk_min_rows else 0
-        if numbers <= 0:
-            return None, 1
-        return torch.empty(int(numbers), dtype=torch.float32, device=device), 1 if small_rows > 0 else 0
+    # Retention in bf16: a request of more rows goes by chunks of 64 rows, any other token by token, whatever the step's
+    # other requests are (both kernels look at each request on the device).  us a call, loop / chunks, one request:
+    #     heads x key x value     65 rows      128      160      192      224      256      384      512      1024
+    #      8 x 128 x 128        20.7/31.0  37.5/43.7  46/43   54/48    63/48    72/51   106/46   140/47   277/51
+    #     16 x 128 x 128        21.1/47.2  37.8/50.9  46/48   55/48    64/47    72/46   107/48   142/50   281/63
+    #     32 x 128 x 128        21.5/52.1  38.8/47.1  48/49   56/49    65/50    74/56   110/59   146/62   290/123
+    #      8 x  64 x  64        14.9/17.7  26.5/18.1    -     38/18      -      50/19    74/21    97/22   191/27
+    # (A step with requests on both sides runs both, one after the other.)
+    chunk_min_rows = 192
+    chunk_scratch_numbers = 1 << 25        # of scratch at most (128 MB; more chunks go in waves)
 
     def diff_qk_prepare(self, qkv: torch.Tensor, *, q_norm, k_norm, eps: float, frequencies, positions, slot_mapping,
                         cache: torch.Tensor, write_kv: bool, heads: int, kv_heads: int, key_dim: int, value_dim: int) -> None:

@@ -67,6 +67,46 @@ def test_retention(dim, vdim, lens):
         assert torch.equal(state[0], first[0]) and torch.equal(state[len(lens) + 1:], first[len(lens) + 1:])
 
 
+def _retention_inputs(T, heads, dim, vdim, slots):
+    g = torch.Generator().manual_seed(T + dim)
+    qk = torch.randn(T, 2 * heads * dim, generator=g).bfloat16().to(DEV)
+    v = torch.randn(T, heads * vdim, generator=g).bfloat16().to(DEV)
+    decay = torch.tensor([0.0, -0.01, -0.97][:heads], device=DEV)
+    return qk, v, decay, torch.randn(slots, heads * dim * vdim, generator=g).to(DEV)
+
+
+@pytest.mark.parametrize("dim, vdim", [(64, 64), (128, 192)])
+def test_retention_by_the_request(dim, vdim):
+    """A request's bits are its own: alone and beside requests on both sides of the rule, in steps whose plans cover any make-up
+    (padded ones), and with scratch for one chunk, for three, or for all of the step's."""
+    from pih_b200.engine.runner import _PaddedPlans
+    ops, heads = _ops(), 3
+    lens = [ops.chunk_min_rows + 1, 40, 700, 1, ops.chunk_min_rows, 65]
+    T, cu = sum(lens), [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    qk, v, decay, first = _retention_inputs(T, heads, dim, vdim, len(lens))
+
+    def run(lo, hi, cu, slots, plans=None, scratch=None):
+        step, state = _step(list(range(hi - lo)), [0] * (hi - lo), cu, slots), first.clone()
+        if plans is not None:
+            step.attention_plans = plans
+        if scratch is not None:
+            ops.chunk_scratch_numbers = scratch * heads * dim * vdim
+        o = ops.retention(qk[lo:hi], v[lo:hi], frequencies=None, decay_minus_one=decay, key_scale=0.25, state=state, step=step,
+                          heads=heads, key_dim=dim, value_dim=vdim)
+        ops.chunk_scratch_numbers = type(ops).chunk_scratch_numbers
+        return o, state
+    together, states = run(0, T, cu, list(range(len(lens))))
+    for kw in (dict(plans=_PaddedPlans(1024, 4096)), dict(scratch=1), dict(scratch=3)):
+        o, state = run(0, T, cu, list(range(len(lens))), **kw)
+        assert torch.equal(o, together) and torch.equal(state, states)
+    for r in range(len(lens)):
+        for plans in (None, _PaddedPlans(1024, 4096)):
+            o, state = run(cu[r], cu[r + 1], [0, lens[r]], [r], plans)
+            assert torch.equal(o, together[cu[r]:cu[r + 1]]) and torch.equal(state[r], states[r])
+
+
 def _delta(ops, T, lens, slots, qkv, beta, a, bias, log, state, dim, vdim, heads, kv_heads):
     cu = [0]
     for n in lens:

@@ -66,9 +66,11 @@ __device__ __forceinline__ void load_rows(float* dst, const float* src, long lon
   }
 }
 
-// The same from bf16, widened on the way (done when the function returns).
+// The same from bf16, widened on the way (done when the function returns).  Says whether one of this thread's numbers is
+// infinite or none.
 template <int COLS, int LD>
-__device__ __forceinline__ void load_rows(float* dst, const __nv_bfloat16* src, long long ld, int rows) {
+__device__ __forceinline__ bool load_rows(float* dst, const __nv_bfloat16* src, long long ld, int rows) {
+  bool wild = false;
   for (int e = threadIdx.x; e < kRows * (COLS / 8); e += blockDim.x) {
     const int row = e / (COLS / 8), c = (e % (COLS / 8)) * 8;
     const uint4 x = row < rows ? *reinterpret_cast<const uint4*>(src + row * ld + c) : make_uint4(0u, 0u, 0u, 0u);
@@ -78,10 +80,12 @@ __device__ __forceinline__ void load_rows(float* dst, const __nv_bfloat16* src, 
     for (int i = 0; i < 4; ++i) {
       f[2 * i] = __uint_as_float(w[i] << 16);
       f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+      wild = wild || (w[i] & 0x7f80u) == 0x7f80u || (w[i] & 0x7f800000u) == 0x7f800000u;
     }
     *reinterpret_cast<float4*>(dst + row * LD + c) = make_float4(f[0], f[1], f[2], f[3]);
     *reinterpret_cast<float4*>(dst + row * LD + c + 4) = make_float4(f[4], f[5], f[6], f[7]);
   }
+  return wild;
 }
 
 // Products of 32-bit numbers in shared memory by 256 threads, (ty, tx) = (thread / 16, thread % 16): rows ty * RM + i.
@@ -115,8 +119,9 @@ __device__ __forceinline__ void clear(float2 (&acc)[R][C]) {
 }
 
 // acc[i][2 g + u] (columns 64 g + 4 tx + 2 u, + 1) += sum over k < K (a multiple of 4) of a[row][k] b[k][column].  Chains of
-// 16 products, whose sums are added up: the rounding error is that of 16 + K / 16 additions, not of K.
-template <int RM, int RN>
+// 16 products, whose sums are added up: the rounding error is that of 16 + K / 16 additions, not of K.  TRIANGLE: without the
+// products of k > row, whose a is zero: the same sums, but what b holds there may be anything.
+template <int RM, int RN, bool TRIANGLE = false>
 __device__ __forceinline__ void multiply_columns(float2 (&acc)[RM][RN / 2], const float* a, int lda, const float* b, int ldb, int K) {
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
 #pragma unroll 1
@@ -139,6 +144,7 @@ __device__ __forceinline__ void multiply_columns(float2 (&acc)[RM][RN / 2], cons
         for (int u = 0; u < 4; ++u)
 #pragma unroll
           for (int g = 0; g < RN / 4; ++g) {
+            if (TRIANGLE && k + u > ty * RM + i) continue;
             const float2 xx = make_float2(xs[u], xs[u]);
             part[i][2 * g] = fma2(xx, make_float2(y[u][g].x, y[u][g].y), part[i][2 * g]);
             part[i][2 * g + 1] = fma2(xx, make_float2(y[u][g].z, y[u][g].w), part[i][2 * g + 1]);

@@ -388,9 +388,10 @@ retention_chunk_out_kernel(const RetentionArgs p) {
       o[i][j].y *= power[ty * 4 + i + 1];
     }
   __syncthreads();
-  chunks::load_rows<VT, VT>(ks, p.v + c.first * p.ldv + static_cast<long long>(h) * p.vdim + v0, p.ldv, c.rows);
-  __syncthreads();
-  chunks::multiply_columns<4, RN>(o, P, LP, ks, VT, (tid >> 5) * 8 + 8);       // (the warp's rows see no later ones)
+  const bool wild = chunks::load_rows<VT, VT>(ks, p.v + c.first * p.ldv + static_cast<long long>(h) * p.vdim + v0, p.ldv, c.rows);
+  const int seen = (tid >> 5) * 8 + 8;                     // (the warp's rows see no later ones)
+  if (!__syncthreads_or(wild)) chunks::multiply_columns<4, RN>(o, P, LP, ks, VT, seen);
+  else chunks::multiply_columns<4, RN, true>(o, P, LP, ks, VT, seen);          // (zero times infinity is not zero)
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int row = ty * 4 + i;

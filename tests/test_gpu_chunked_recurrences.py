@@ -107,6 +107,33 @@ def test_retention_by_the_request(dim, vdim):
             assert torch.equal(o, together[cu[r]:cu[r + 1]]) and torch.equal(state[r], states[r])
 
 
+@pytest.mark.parametrize("dim, vdim", [(64, 64), (128, 128)])
+@pytest.mark.parametrize("row", [0, 66, 127, 200, 228])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_retention_before_a_wild_row(dim, vdim, row, value):
+    """A value or a key that is infinite or no number reaches its own row and later ones: the bits of earlier rows, and of its
+    own row's other columns, stay."""
+    ops, heads, T = _ops(), 2, 229
+    assert T > ops.chunk_min_rows
+    qk, v, decay, first = _retention_inputs(T, heads, dim, vdim, 1)
+
+    def run(qk, v):
+        state = first.clone()
+        return ops.retention(qk, v, frequencies=None, decay_minus_one=decay, key_scale=0.25, state=state,
+                             step=_step(list(range(T)), [0] * T, [0, T], [0]), heads=heads, key_dim=dim, value_dim=vdim), state
+    (plain, state), spoilt = run(qk, v), v.clone()
+    spoilt[row, 5] = value                                                      # head 0, column 5
+    o, after = run(qk, spoilt)
+    same = torch.ones_like(plain, dtype=torch.bool)
+    same[row:, 0, 5] = False
+    assert torch.equal(o[same], plain[same]) and not bool(o[row:, 0, 5].isfinite().any())
+    assert torch.equal(after.view(heads, dim, vdim)[1], state.view(heads, dim, vdim)[1])
+    spoilt = qk.clone()
+    spoilt[row, heads * dim + 3] = value                                        # the key of head 0
+    o, _ = run(spoilt, v)
+    assert torch.equal(o[:row], plain[:row]) and torch.equal(o[:, 1], plain[:, 1]) and not bool(o[row:, 0].isfinite().any())
+
+
 def _delta(ops, T, lens, slots, qkv, beta, a, bias, log, state, dim, vdim, heads, kv_heads):
     cu = [0]
     for n in lens:

@@ -231,21 +231,52 @@ __device__ __forceinline__ void f32_attend(const F32AttentionArgs& a, float* sme
     }
     __syncwarp();
     const int count = min(32, last - 32 * tile + 1);
+    auto value = [&](int jj, float (&v)[C]) {              // of key jj of the tile, this lane's columns
+      const long long from = __shfl_sync(0xffffffffu, mine, jj);
+      const float* vrow = a.cache + from + to_values + lane * C;
+      if (C == 4) {
+        const float4 x = from >= 0 ? *reinterpret_cast<const float4*>(vrow) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        v[0] = x.x; v[1] = x.y; v[C - 2] = x.z; v[C - 1] = x.w;
+      } else {
+        const float2 x = from >= 0 ? *reinterpret_cast<const float2*>(vrow) : make_float2(0.0f, 0.0f);
+        v[0] = x.x; v[1] = x.y;
+      }
+    };
+    // Keys that some of the rows do not see, later rows' or behind a window, enter with a weight of zero, and zero times
+    // infinity is not zero: such a tile's values are looked through first, and if not all are finite each row takes its own.
+    bool wild = false;
+    if (last > p0 && (32 * tile + 31 > p0 || (a.window > 0 && 32 * tile <= last - a.window))) {
+      float zeros = 0.0f;
+#pragma unroll 8
+      for (int jj = 0; jj < count; ++jj) {
+        float v[C];
+        value(jj, v);
+#pragma unroll
+        for (int c = 0; c < C; ++c) zeros = fmaf(v[c], 0.0f, zeros);
+      }
+      wild = __any_sync(0xffffffffu, zeros != 0.0f);
+    }
+    if (wild) {
+#pragma unroll 1
+      for (int jj = 0; jj < count; ++jj) {
+        const int key = 32 * tile + jj;
+        float v[C];
+        value(jj, v);
+#pragma unroll
+        for (int i = 0; i < P; ++i) {
+          const int p = p0 + i / group;
+          if (key > p || (a.window > 0 && key <= p - a.window)) continue;
+#pragma unroll
+          for (int c = 0; c < C; ++c) acc[i][c] = fmaf(ps[i * 32 + jj], v[c], acc[i][c]);
+        }
+      }
+      continue;
+    }
 #pragma unroll 2
     for (int jj = 0; jj < count; jj += 4) {
       float v[4][C];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const long long from = __shfl_sync(0xffffffffu, mine, jj + u);
-        const float* vrow = a.cache + from + to_values + lane * C;
-        if (C == 4) {
-          const float4 x = from >= 0 ? *reinterpret_cast<const float4*>(vrow) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          v[u][0] = x.x; v[u][1] = x.y; v[u][C - 2] = x.z; v[u][C - 1] = x.w;
-        } else {
-          const float2 x = from >= 0 ? *reinterpret_cast<const float2*>(vrow) : make_float2(0.0f, 0.0f);
-          v[u][0] = x.x; v[u][1] = x.y;
-        }
-      }
+      for (int u = 0; u < 4; ++u) value(jj + u, v[u]);
 #pragma unroll
       for (int i = 0; i < P; ++i) {
         const float4 w = *reinterpret_cast<const float4*>(ps + i * 32 + jj);

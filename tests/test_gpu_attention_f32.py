@@ -46,3 +46,28 @@ def test_rows_of_padding_and_keys_without_a_page(ops):
     with pytest.raises(Exception):
         ops.check_errors()
     ops.clear_errors()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("heads,kv_heads", [(4, 4), (4, 2), (16, 1)])
+@pytest.mark.parametrize("n,window", [(40, None), (17, None), (150, 20), (33, 1)])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_values_that_a_row_does_not_see(ops, D, heads, kv_heads, n, window, value):
+    """A value that is infinite or no number reaches the rows that see its key; the bits of earlier rows of the same blocks, and
+    of rows whose window has left it behind, stay."""
+    s = _paged_setup(torch.float32, [n], [n], heads, kv_heads, D, 16, seed=n)
+    whole = _run(ops, s, slice(None), heads, kv_heads, D, window)
+    kinds = {"value": 1} if value != value else {"value": 1, "key": 0}        # (a key of NaN or infinity spoils its rows' sums)
+    for at in {0, 5, n // 2, n - 1}:
+        for kind in kinds.values():
+            page = int(s["table"][0, at // 16])
+            kept = s["cache"][page, kind, 0, at % 16, 3].clone()
+            s["cache"][page, kind, 0, at % 16, 3] = value
+            got = _run(ops, s, slice(None), heads, kv_heads, D, window)
+            s["cache"][page, kind, 0, at % 16, 3] = kept
+            blind = [t for t in range(n) if t < at or (window and t >= at + window)]
+            assert torch.equal(got[blind], whole[blind])
+            if kind == 1:
+                sees = [t for t in range(n) if t not in blind]
+                assert not bool(got[sees][:, 3].isfinite().any())
+            ops.clear_errors()

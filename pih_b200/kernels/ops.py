@@ -731,7 +731,13 @@ class CudaOps:
 
     latent_mma = True                      # bf16 attention over a latent of rank 64 ... 512: the tensor-core kernel ...
     latent_mma_min_rows = 0                # ... for steps of more rows than this
-    latent_mma_rows_above = 64             # ... with blocks of 4 or 8 rows of a request from this many rows on
+    latent_mma_rows_above = 64             # ... with blocks of 4 rows of a request from more rows than this on, and of 8
+    # from more than this on: half the blocks with twice the work are slower until they fill the GPU.  us, 4 / 8 rows a block:
+    #     heads, rank     128 rows     300        384        512        768        1024       2048
+    #     8, 64           15.9/21.5  15.5/20.7  17.5/20.6  22.6/21.2  42.5/26.4  54.2/34.6   90/68
+    #     8, 256          22.5/34.1  33.7/42.4  42.8/44.3  55.9/51.2  92.3/75.3   130/93    279/172
+    #     8, 512          31.0/36.9  52.1/51.4  63.8/63.2  94.3/77.7   163/122    241/178   598/373
+    latent_pairs_rows_above = 448
     latent_split = True                    # bf16 attention over a latent: keys cut into parts (False: the in-order kernel)
     batched_library_min_rows = 128         # bf16 batched products of at least this many rows are the library's
 
@@ -985,7 +991,7 @@ class CudaOps:
             # a row's keys are cut into ``splits`` parts side by side, and each of a block's 8 warps is a part of its own
             # steps of many rows (prompt portions): a block is 4 consecutive rows of a request, which share a tile, or 8
             # of at most 8 heads, two rows of which fill an MMA
-            per_block = (8 if heads <= 8 else 4) if T > self.latent_mma_rows_above else 1
+            per_block = 1 if T <= self.latent_mma_rows_above else (8 if heads <= 8 and T > self.latent_pairs_rows_above else 4)
             blocks = (T if per_block == 1 else -(-T // per_block) + step.num_requests) * (-(-heads // 16)) * (2 if rank > 256 else 1)
             splits = max(1, min(16, (2 * 148) // max(1, blocks)))
             parts = splits * (8 if per_block == 1 else 2)

@@ -9,10 +9,28 @@ from test_gpu_rigotar import DEV
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture
+def pairs(request):
+    """The number of rows above which two rows fill an MMA: as it is, or none."""
+    from pih_b200.kernels import get_ops
+    ops = get_ops(torch.device(DEV))
+    if request.param:
+        ops.latent_pairs_rows_above = 0
+    yield
+    ops.latent_pairs_rows_above = type(ops).latent_pairs_rows_above
+
+
+@pytest.mark.parametrize("pairs", [False, True], indirect=True)
 @pytest.mark.parametrize("rank, heads", [(256, 8), (256, 7), (192, 1), (512, 8), (64, 8), (256, 9), (256, 16)])
-def test_portions_of_several_requests(rank, heads):
+def test_portions_of_several_requests(rank, heads, pairs):
     """Blocks of one tile each (contexts of up to 371 keys in 5 to 10 splits)."""
     rigotar.test_latent_attention_portions_of_several_requests(rank, heads)
+
+
+@pytest.mark.parametrize("rows", [64, 65, 448, 449])
+def test_where_the_rows_of_a_block_change(rows):
+    """1, 4 and 8 rows a block, at both sides of the rule."""
+    test_contexts_of_many_tiles(0, rows, 64, 2, 0)
 
 
 def _plain_windowed(q, lat, positions, window, scale):
@@ -27,11 +45,11 @@ def _plain_windowed(q, lat, positions, window, scale):
     return out
 
 
-# 1500 to 1507 rows: one split, a block's tiles are 9 with the window and up to 12 without.  301 rows behind 3700: without a
-# window 7 splits of 5 tiles (8 rows a block) or 3 of 11 (4 rows), with it 2 and 3 tiles.  The last one is seldom whole.
+# 1500 to 1507 rows: one split, a block's tiles are 9 with the window and up to 12 without.  301 and 501 rows behind 3700: 3
+# splits of 11 tiles (4 rows a block), 4 of 9 (8 rows) or 2 of 17; with the window 2 to 5 tiles.  The last is seldom whole.
 @pytest.mark.parametrize("window", [0, 1024])
 @pytest.mark.parametrize("rank, heads", [(64, 8), (128, 7), (192, 8), (256, 8), (256, 16)])
-@pytest.mark.parametrize("past, rows", [(0, n) for n in range(1500, 1508)] + [(3700, 301)])
+@pytest.mark.parametrize("past, rows", [(0, n) for n in range(1500, 1508)] + [(3700, 301), (3700, 501)])
 def test_contexts_of_many_tiles(past, rows, rank, heads, window):
     """Rows of a request over more tiles than there are buffers, all remainders of rows in the last block: its warps without
     a row run ahead of the others, which must still see every key of their tile.  16 lost keys of 1024 are an eighth of a row."""

@@ -94,11 +94,11 @@ __device__ __forceinline__ uint32_t load_u32_from_block(const uint32_t* local, u
 // The prefixes are looked for among buckets of scaled values first: kBuckets equal steps from the row's maximum down to
 // its minimum, or 31 below the maximum if that is nearer (a mass is zero from 30.5 on), with the count and the mass of
 // each.  Every wanted prefix ends inside one bucket, whose elements — a few hundred of 150 000 — are collected and ranked
-// one by one.  So a row takes two passes with arithmetic (maximum, buckets) and one of comparisons for each prefix, where
+// one by one (a top_k that ends behind all mass leaves out nothing).  So a row takes two passes with arithmetic (maximum, buckets) and one of comparisons for each prefix, where
 // radix passes alone (find_crossing: four for each prefix with an exponential an element, then the ties) took 147 us for
 // 32 rows of 151 936, this 55 to 65 us (one row: 27 us, and 5 to 10 us more for each of top_k and top_p).  They remain
-// for rows whose crossing falls into a bucket of more than kListed elements (many equal logits, a top_k beyond 31), and
-// for rows with a value that is not finite.
+// for rows with a value that is not finite, and where a bucket holds too many elements that are not all equal, also after
+// the buckets have divided what one of them held (one logit far above a narrow bulk).
 constexpr int kBuckets = 1984, kOwned = kBuckets / kSampleCluster, kBucketRange = 31;
 constexpr int kListed = 1024, kListedHere = 512;
 
@@ -123,6 +123,7 @@ struct SampleShared {
   uint32_t owned_count[kOwned];                          // buckets rank * kOwned ...: the row's
   unsigned long long rank_count[kSampleCluster], rank_mass[kSampleCluster];   // and the sums of every rank's
   int listed;
+  uint32_t key_range[2];                                 // the lowest and highest key of a bucket
   unsigned long long won[3];                             // the element that was found, count and mass up to it
   unsigned long long ghist[256];                         // the row's
   unsigned long long mine[2][kExchangeWords];            // this block's words of an exchange, two in turn
@@ -223,6 +224,111 @@ __device__ unsigned long long prefix_total(SampleShared& sm, RowView& rv, const 
   for (int r = 0; r < kSampleCluster; ++r) total += sm.all[r][0];
   __syncthreads();
   return total;
+}
+
+// The place among the members of ``p`` with exactly this key where the running total, ``acc`` in front of them, reaches the
+// target: ties have one weight and follow one another by their ids.  ``upto`` (if not null): the total up to and with it.
+__device__ Prefix find_among_ties(SampleShared& sm, RowView& rv, const Prefix& p, bool use_mass, uint32_t key_c,
+                                  unsigned long long acc, unsigned long long target, unsigned long long* upto) {
+  // members with exactly this key share one weight; how many of them are needed.  Ties are counted in id order:
+  // a thread takes a run of consecutive ids of this block's part, and the blocks' parts follow one another.
+  const int span = rv.hi - rv.lo;
+  const int chunk = (span + blockDim.x - 1) / blockDim.x;
+  const int lo = rv.lo + threadIdx.x * chunk, hi = min(rv.hi, lo + chunk);
+  int mine = 0;
+  unsigned long long a0 = 1ull;
+  for (int id = lo; id < hi; ++id) {
+    if (!allowed(rv, id)) continue;
+    const float s = scaled_of(rv, id);
+    const uint32_t key = ordered_key(s);
+    if (key == key_c && member(p, key, id)) {
+      ++mine;
+      if (use_mass) a0 = mass_of(rv, s);
+    }
+  }
+  // exclusive scan of `mine` over the block, in thread order
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int incl = mine;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int n = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += n;
+  }
+  __syncthreads();
+  if (lane == 31) sm.iscratch[warp] = incl;
+  if (threadIdx.x == 0) sm.a0 = 0ull;
+  __syncthreads();
+  if (warp == 0) {
+    int w = lane < (blockDim.x >> 5) ? sm.iscratch[lane] : 0;
+    int wi = w;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int n = __shfl_up_sync(0xffffffffu, wi, d);
+      if (lane >= d) wi += n;
+    }
+    sm.iscratch[lane] = wi - w;          // exclusive prefix of the warp totals
+    if (lane == 31) sm.iscratch[32] = wi;  // this block's ties
+  }
+  __syncthreads();
+  const int before_in_block = sm.iscratch[warp] + incl - mine;
+  const int block_ties = sm.iscratch[32];
+  if (mine > 0 && before_in_block == 0) sm.a0 = a0;       // (every tie has the same weight)
+  __syncthreads();
+  {
+    const unsigned long long w[kExchangeWords] = {static_cast<unsigned long long>(block_ties), sm.a0, 0ull, 0ull};
+    exchange(sm, rv, w);
+  }
+  int ties = 0, before_block = 0;
+  unsigned long long w0 = 1ull;
+  bool have = false;
+#pragma unroll
+  for (int r = 0; r < kSampleCluster; ++r) {
+    const int t = static_cast<int>(sm.all[r][0]);
+    if (static_cast<uint32_t>(r) < rv.rank) before_block += t;
+    if (t > 0 && !have) {
+      w0 = sm.all[r][1];
+      have = true;
+    }
+    ties += t;
+  }
+  if (!use_mass) w0 = 1ull;
+  // every tie has weight w0 (> 0 where mass is used: a zero weight cannot reach the target)
+  unsigned long long need = w0 ? (target - acc + w0 - 1) / w0 : 1ull;
+  if (need < 1) need = 1;
+  if (need > static_cast<unsigned long long>(ties)) need = ties;
+  const int r = static_cast<int>(need);               // the r-th tie in id order, 1-based
+  if (upto != nullptr) *upto = acc + need * w0;
+  const int before = before_block + before_in_block;
+  if (threadIdx.x == 0) sm.found = -1;
+  __syncthreads();
+  if (mine > 0 && before < r && r <= before + mine) {
+    int seen = before;
+    for (int id = lo; id < hi; ++id) {
+      if (!allowed(rv, id)) continue;
+      const uint32_t key = ordered_key(scaled_of(rv, id));
+      if (key == key_c && member(p, key, id)) {
+        if (++seen == r) {
+          sm.found = id;
+          break;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  {
+    const unsigned long long w[kExchangeWords] = {static_cast<unsigned long long>(static_cast<long long>(sm.found)), 0ull, 0ull, 0ull};
+    exchange(sm, rv, w);
+  }
+  Prefix out;
+  out.key = key_c;
+  out.id = 0;
+#pragma unroll
+  for (int q = 0; q < kSampleCluster; ++q) {
+    const long long f = static_cast<long long>(sm.all[q][0]);
+    if (f >= 0) out.id = static_cast<int>(f);
+  }
+  __syncthreads();
+  return out;
 }
 
 // First place, in sorted order among the members of `p`, where the running total (count or mass) reaches a target
@@ -339,104 +445,7 @@ __device__ Prefix find_crossing(SampleShared& sm, RowView& rv, const Prefix& p, 
   }
   const uint32_t key_c = sm.prefix_val;
   const unsigned long long acc = sm.acc;
-  // members with exactly this key share one weight; how many of them are needed.  Ties are counted in id order:
-  // a thread takes a run of consecutive ids of this block's part, and the blocks' parts follow one another.
-  const int span = rv.hi - rv.lo;
-  const int chunk = (span + blockDim.x - 1) / blockDim.x;
-  const int lo = rv.lo + threadIdx.x * chunk, hi = min(rv.hi, lo + chunk);
-  int mine = 0;
-  unsigned long long a0 = 1ull;
-  for (int id = lo; id < hi; ++id) {
-    if (!allowed(rv, id)) continue;
-    const float s = scaled_of(rv, id);
-    const uint32_t key = ordered_key(s);
-    if (key == key_c && member(p, key, id)) {
-      ++mine;
-      if (use_mass) a0 = mass_of(rv, s);
-    }
-  }
-  // exclusive scan of `mine` over the block, in thread order
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int incl = mine;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const int n = __shfl_up_sync(0xffffffffu, incl, d);
-    if (lane >= d) incl += n;
-  }
-  __syncthreads();
-  if (lane == 31) sm.iscratch[warp] = incl;
-  if (threadIdx.x == 0) sm.a0 = 0ull;
-  __syncthreads();
-  if (warp == 0) {
-    int w = lane < (blockDim.x >> 5) ? sm.iscratch[lane] : 0;
-    int wi = w;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const int n = __shfl_up_sync(0xffffffffu, wi, d);
-      if (lane >= d) wi += n;
-    }
-    sm.iscratch[lane] = wi - w;          // exclusive prefix of the warp totals
-    if (lane == 31) sm.iscratch[32] = wi;  // this block's ties
-  }
-  __syncthreads();
-  const int before_in_block = sm.iscratch[warp] + incl - mine;
-  const int block_ties = sm.iscratch[32];
-  if (mine > 0 && before_in_block == 0) sm.a0 = a0;       // (every tie has the same weight)
-  __syncthreads();
-  {
-    const unsigned long long w[kExchangeWords] = {static_cast<unsigned long long>(block_ties), sm.a0, 0ull, 0ull};
-    exchange(sm, rv, w);
-  }
-  int ties = 0, before_block = 0;
-  unsigned long long w0 = 1ull;
-  bool have = false;
-#pragma unroll
-  for (int r = 0; r < kSampleCluster; ++r) {
-    const int t = static_cast<int>(sm.all[r][0]);
-    if (static_cast<uint32_t>(r) < rv.rank) before_block += t;
-    if (t > 0 && !have) {
-      w0 = sm.all[r][1];
-      have = true;
-    }
-    ties += t;
-  }
-  if (!use_mass) w0 = 1ull;
-  // every tie has weight w0 (> 0 where mass is used: a zero weight cannot reach the target)
-  unsigned long long need = w0 ? (target - acc + w0 - 1) / w0 : 1ull;
-  if (need < 1) need = 1;
-  if (need > static_cast<unsigned long long>(ties)) need = ties;
-  const int r = static_cast<int>(need);               // the r-th tie in id order, 1-based
-  const int before = before_block + before_in_block;
-  if (threadIdx.x == 0) sm.found = -1;
-  __syncthreads();
-  if (mine > 0 && before < r && r <= before + mine) {
-    int seen = before;
-    for (int id = lo; id < hi; ++id) {
-      if (!allowed(rv, id)) continue;
-      const uint32_t key = ordered_key(scaled_of(rv, id));
-      if (key == key_c && member(p, key, id)) {
-        if (++seen == r) {
-          sm.found = id;
-          break;
-        }
-      }
-    }
-  }
-  __syncthreads();
-  {
-    const unsigned long long w[kExchangeWords] = {static_cast<unsigned long long>(static_cast<long long>(sm.found)), 0ull, 0ull, 0ull};
-    exchange(sm, rv, w);
-  }
-  Prefix out;
-  out.key = key_c;
-  out.id = 0;
-#pragma unroll
-  for (int q = 0; q < kSampleCluster; ++q) {
-    const long long f = static_cast<long long>(sm.all[q][0]);
-    if (f >= 0) out.id = static_cast<int>(f);
-  }
-  __syncthreads();
-  return out;
+  return find_among_ties(sm, rv, p, use_mass, key_c, acc, target, nullptr);
 }
 
 // This rank's running totals from the largest bucket down: warp 0 finds the first of its buckets where the running total
@@ -480,16 +489,26 @@ __device__ void find_owned(SampleShared& sm, uint32_t rank, bool use_mass, unsig
   }
 }
 
-// Where the search stands: the bucket whose elements are listed (-1: none), the count and mass in front of it, the
-// elements, and the mass up to the last prefix that was found.
+__device__ __forceinline__ float scaled_of_key(uint32_t key) {   // ordered_key's other way
+  return __uint_as_float((key & 0x80000000u) ? key ^ 0x80000000u : ~key);
+}
+
+// Where the search stands: the stretch of scaled values that the buckets divide (the whole row's, or what one bucket of it
+// held), the count and mass in front of it; the bucket whose elements are listed (-1: none), the count and mass in front of
+// it, the elements; and the mass up to the last prefix that was found.
 struct Buckets {
-  float per_unit;
+  float per_unit_of_row;
+  float top, floor, per_unit;
+  bool divided;                                            // (a bucket of the row's, not the row)
+  unsigned long long count_base, mass_base;
   int listed_bucket, elements;
   unsigned long long count_before, mass_before, mass_upto;
 };
 
-__device__ __forceinline__ int bucket_of(const RowView& rv, const Buckets& bk, float scaled) {
-  return min(kBuckets - 1, static_cast<int>((rv.max_scaled - scaled) * bk.per_unit));
+// (negative: outside of the stretch, or a suppressed id above the row's)
+__device__ __forceinline__ int bucket_of(const Buckets& bk, float scaled) {
+  if (bk.divided && (scaled > bk.top || scaled < bk.floor)) return -1;
+  return min(kBuckets - 1, static_cast<int>((bk.top - scaled) * bk.per_unit));
 }
 
 // The counts and masses of all buckets.
@@ -499,7 +518,8 @@ __device__ void fill_buckets(SampleShared& sm, RowView& rv, Buckets& bk) {
   for (int id = rv.lo + threadIdx.x; id < rv.hi; id += blockDim.x) {
     if (!allowed(rv, id)) continue;
     const float s = rv.staged[id - rv.lo];
-    const int b = bucket_of(rv, bk, s);
+    const int b = bucket_of(bk, s);
+    if (bk.divided && b < 0) continue;
     const unsigned long long a = mass_of(rv, s);
     const uint32_t a0 = static_cast<uint32_t>(a) & 0x7FFFu, a1 = static_cast<uint32_t>(a >> 15) & 0x7FFFu,
                    a2 = static_cast<uint32_t>(a >> 30);
@@ -531,16 +551,25 @@ __device__ void fill_buckets(SampleShared& sm, RowView& rv, Buckets& bk) {
     sm.rank_count[threadIdx.x] = sm.all[threadIdx.x][0];
     sm.rank_mass[threadIdx.x] = sm.all[threadIdx.x][1];
   }
+  bk.listed_bucket = -1;
   __syncthreads();
-  bk.mass_upto = 0;
-  for (int r = 0; r < kSampleCluster; ++r) bk.mass_upto += sm.rank_mass[r];
+}
+
+// Buckets over the whole row.
+__device__ void fill_row(SampleShared& sm, RowView& rv, Buckets& bk) {
+  bk.top = rv.max_scaled;
+  bk.per_unit = bk.per_unit_of_row;
+  bk.divided = false;
+  bk.count_base = bk.mass_base = 0ull;
+  fill_buckets(sm, rv, bk);
 }
 
 // The first place where the running total reaches target (count or mass; at most the total up to the last prefix found);
 // false: its bucket holds too many elements.  All blocks of the cluster find the same.
 __device__ bool find_in_buckets(SampleShared& sm, RowView& rv, Buckets& bk, bool use_mass, unsigned long long target, Prefix* out) {
-  if (bk.listed_bucket < 0 || !use_mass || target <= bk.mass_before) {
-    unsigned long long count = 0, mass = 0;
+  if (use_mass && target <= bk.mass_base) fill_row(sm, rv, bk);          // (in front of the bucket that was divided)
+  while (bk.listed_bucket < 0 || !use_mass || target <= bk.mass_before) {
+    unsigned long long count = bk.count_base, mass = bk.mass_base;
     int owner = -1;
     for (int r = 0; r < kSampleCluster; ++r) {
       const unsigned long long c = sm.rank_count[r], m = sm.rank_mass[r];
@@ -553,7 +582,11 @@ __device__ bool find_in_buckets(SampleShared& sm, RowView& rv, Buckets& bk, bool
     }
     if (owner < 0) return false;
     if (rv.rank == static_cast<uint32_t>(owner) && threadIdx.x < 32) find_owned(sm, rv.rank, use_mass, target, count, mass);
-    if (threadIdx.x == 0) sm.listed = 0;
+    if (threadIdx.x == 0) {
+      sm.listed = 0;
+      sm.key_range[0] = 0xffffffffu;
+      sm.key_range[1] = 0u;
+    }
     __syncthreads();
     {
       const unsigned long long w[kExchangeWords] = {sm.won[0], sm.won[1], sm.won[2], 0ull};
@@ -562,10 +595,10 @@ __device__ bool find_in_buckets(SampleShared& sm, RowView& rv, Buckets& bk, bool
     const int b = static_cast<int>(sm.all[owner][0]);
     bk.count_before = sm.all[owner][1];
     bk.mass_before = sm.all[owner][2];
-    bk.listed_bucket = b;
+    if (!use_mass && bk.mass_before == bk.mass_upto) return true;      // (mass_upto: the row's, a count is asked for first)
     for (int id = rv.lo + threadIdx.x; id < rv.hi; id += blockDim.x) {
       const float s = rv.staged[id - rv.lo];
-      if (bucket_of(rv, bk, s) != b || !allowed(rv, id)) continue;
+      if (bucket_of(bk, s) != b || !allowed(rv, id)) continue;
       const int at = atomicAdd(&sm.listed, 1);
       if (at < kListedHere)
         sm.list.here[at] = (static_cast<unsigned long long>(~ordered_key(s)) << 32) | static_cast<uint32_t>(id);
@@ -581,17 +614,58 @@ __device__ bool find_in_buckets(SampleShared& sm, RowView& rv, Buckets& bk, bool
       fits = fits && sm.all[r][0] <= static_cast<unsigned long long>(kListedHere);
       n += static_cast<int>(sm.all[r][0]);
     }
-    if (!fits || n > kListed) return false;                // (before anything is written where the radix passes count)
+    if (!fits || n > kListed) {                            // too many: if they are all equal, their ids decide
+      bk.listed_bucket = -1;
+      uint32_t low = 0xffffffffu, high = 0u;
+      for (int id = rv.lo + threadIdx.x; id < rv.hi; id += blockDim.x) {
+        const float s = rv.staged[id - rv.lo];
+        if (bucket_of(bk, s) != b || !allowed(rv, id)) continue;
+        low = min(low, ordered_key(s));
+        high = max(high, ordered_key(s));
+      }
+      low = __reduce_min_sync(0xffffffffu, low);
+      high = __reduce_max_sync(0xffffffffu, high);
+      if ((threadIdx.x & 31) == 0) {
+        atomicMin(&sm.key_range[0], low);
+        atomicMax(&sm.key_range[1], high);
+      }
+      __syncthreads();
+      const unsigned long long w[kExchangeWords] = {sm.key_range[0], sm.key_range[1], 0ull, 0ull};
+      exchange(sm, rv, w);
+      for (int r = 0; r < kSampleCluster; ++r) {
+        low = min(low, static_cast<uint32_t>(sm.all[r][0]));
+        high = max(high, static_cast<uint32_t>(sm.all[r][1]));
+      }
+      __syncthreads();
+      if (low == high) {
+        unsigned long long upto;
+        const Prefix everything = {0u, 0x7fffffff};        // (the target lies no further than the last prefix found)
+        *out = find_among_ties(sm, rv, everything, use_mass, low, use_mass ? bk.mass_before : bk.count_before, target, &upto);
+        bk.mass_upto = use_mass ? upto : bk.mass_before + (target - bk.count_before) * mass_of(rv, scaled_of_key(low));
+        return true;
+      }
+      // else the buckets divide what this one held, once
+      if (bk.divided) return false;                        // (before anything is written where the radix passes count)
+      bk.top = scaled_of_key(high);
+      bk.floor = scaled_of_key(low);
+      bk.divided = true;
+      bk.per_unit = static_cast<float>(kBuckets - 1) / (bk.top - bk.floor);
+      bk.count_base = bk.count_before;
+      bk.mass_base = bk.mass_before;
+      fill_buckets(sm, rv, bk);
+      continue;
+    }
+    bk.listed_bucket = b;
     for (int r = 0, at = 0; r < kSampleCluster; at += static_cast<int>(sm.all[r][0]), ++r) {
       for (int i = threadIdx.x; i < static_cast<int>(sm.all[r][0]); i += blockDim.x) {
         const unsigned long long o = load_u64_from_block(&sm.list.here[i], r);
-        const uint32_t key = ~static_cast<uint32_t>(o >> 32);
-        const float s = __uint_as_float((key & 0x80000000u) ? key ^ 0x80000000u : ~key);
+        const float s = scaled_of_key(~static_cast<uint32_t>(o >> 32));
         sm.list.order[at + i] = o;
         sm.list.mass[at + i] = mass_of(rv, s);
       }
     }
     bk.elements = n;
+    break;
   }
   __syncthreads();
   // a warp an element, the elements shared out among the blocks: the count and mass up to and with it
@@ -776,10 +850,11 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
                                     (static_cast<uint64_t>(static_cast<uint32_t>(ip[4])) << 32) |
                                         static_cast<uint32_t>(ip[3]));
   const double u = (static_cast<double>(word) + 0.5) / 4294967296.0;
-  Buckets bk = {0.0f, -1, 0, 0ull, 0ull, 0ull};
+  Buckets bk = {};
   if (by_buckets) {
-    bk.per_unit = static_cast<float>(kBuckets - 1) / fmaxf(fminf(best - least, static_cast<float>(kBucketRange)), 1e-6f);
-    fill_buckets(sm, rv, bk);
+    bk.per_unit_of_row = static_cast<float>(kBuckets - 1) / fmaxf(fminf(best - least, static_cast<float>(kBucketRange)), 1e-6f);
+    fill_row(sm, rv, bk);
+    for (int r = 0; r < kSampleCluster; ++r) bk.mass_upto += sm.rank_mass[r];
   }
   if (top_k > 0 && top_k < n_allowed) {
     by_buckets = by_buckets && find_in_buckets(sm, rv, bk, false, static_cast<unsigned long long>(top_k), &kept);

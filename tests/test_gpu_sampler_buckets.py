@@ -17,7 +17,7 @@ def ops():
 
 
 @pytest.mark.parametrize("vocab", [7, 1983, 32768, 151936])
-@pytest.mark.parametrize("shape", ["normal", "equal", "two plateaus", "far apart", "one high"])
+@pytest.mark.parametrize("shape", ["normal", "equal", "two plateaus", "far apart", "one high", "levels", "levels and masked", "cold", "narrow", "very narrow"])
 def test_choices(ops, vocab, shape):
     g = torch.Generator().manual_seed(vocab)
     logits = torch.randn(12, vocab, generator=g) * 2.5
@@ -27,6 +27,15 @@ def test_choices(ops, vocab, shape):
         logits = torch.where(logits > 0.1, 4.0, -1.0)
     if shape == "far apart":                                     # most masses are zero; a top_k ends among them
         logits *= 100.0
+    if shape.startswith("levels"):                               # of a quarter each; more equal values than a list holds
+        logits = torch.round(logits * 2) / 4
+    if shape == "levels and masked":
+        logits[:, ::3] = -1e9
+    if shape == "cold":                                          # as 0.1 would make of them: a top_k ends beyond all mass
+        logits *= 10.0
+    if shape.endswith("narrow"):                                 # one logit above a bulk: more in a bucket than a list holds
+        logits *= 0.12 if shape == "narrow" else 1e-4
+        logits[:, vocab // 2] = 12.0
     if shape == "one high":
         logits[:, vocab // 2] = 60.0
     rows = [([0.7, 1.0, 2.0][i % 3], [1.0, 0.9, 0.3, 1.0][i % 4], [None, 1, 40, vocab // 2 + 1][i % 4], 5 + i, i,

@@ -16,6 +16,7 @@
 // q is read from the fused projection buffer [rows, row_stride] (head h at
 // column h * head_dim); cache layout [page][2][kv_head][page_size][head_dim].
 #include "common.cuh"
+#include "mma.cuh"
 
 namespace pih {
 
@@ -122,11 +123,6 @@ constexpr size_t f32_attention_bytes() {
   return sizeof(float) * (kF32Warps * 32 * (HD + 4) + kF32Pairs * HD + kF32Warps * kF32Pairs * 34);
 }
 
-__device__ __forceinline__ void copy_16_or_zero(void* dst, const void* src, bool there) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
-               "l"(src), "r"(there ? 16 : 0));
-}
-
 struct F32AttentionArgs {
   const float* q;
   int q_stride;
@@ -179,7 +175,7 @@ __device__ __forceinline__ void f32_attend(const F32AttentionArgs& a, float* sme
     for (int jj = 0; jj < 32; jj += 32 / kLanes) {
       const int key = jj + lane / kLanes;
       const long long from = __shfl_sync(0xffffffffu, at, key);
-      copy_16_or_zero(ks + key * LD + (lane % kLanes) * 4, a.cache + (from < 0 ? 0 : from) + (lane % kLanes) * 4, from >= 0);
+      mma::copy_async_16_or_zero(ks + key * LD + (lane % kLanes) * 4, a.cache + (from < 0 ? 0 : from) + (lane % kLanes) * 4, from >= 0);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };

@@ -1,7 +1,8 @@
-// Chunks of 64 rows of the requests of a step, for a recurrence that takes a long request's rows chunk by chunk.
+// Chunks of 64 rows of the requests of a step, for recurrences that take a long request's rows chunk by chunk.
 #pragma once
 
 #include "common.cuh"
+#include "mma.cuh"
 
 namespace pih {
 namespace chunks {
@@ -50,18 +51,12 @@ inline long long at_most(long long rows, int requests, int small_rows) {
   return rows / kRows + (ends < requests ? ends : requests);
 }
 
-__device__ __forceinline__ void copy_async_16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src));
-}
-__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
 // `rows` rows of COLS 32-bit numbers (row stride ld) into shared memory [64][LD] by copies (not waited for), zeros beyond.
 template <int COLS, int LD>
 __device__ __forceinline__ void load_rows(float* dst, const float* src, long long ld, int rows) {
   for (int e = threadIdx.x; e < kRows * (COLS / 4); e += blockDim.x) {
     const int row = e / (COLS / 4), c = (e % (COLS / 4)) * 4;
-    if (row < rows) copy_async_16(dst + row * LD + c, src + row * ld + c);
+    if (row < rows) mma::copy_async_16(dst + row * LD + c, src + row * ld + c);
     else *reinterpret_cast<float4*>(dst + row * LD + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   }
 }

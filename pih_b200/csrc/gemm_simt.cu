@@ -13,6 +13,7 @@
 // (src/backend/cuda/gemm_plan.cpp:83-199: row-major A[m,k], W[n,k] with
 // CUBLAS_OP_T, 32-bit compute); it has no kernel of its own for them.
 #include "common.cuh"
+#include "mma.cuh"
 
 namespace pih {
 
@@ -108,11 +109,6 @@ constexpr size_t tile_bytes() {
   return sizeof(float) * static_cast<size_t>(STAGES) * (ROWS + kTileN) * kTileLd;
 }
 
-__device__ __forceinline__ void copy_16_or_zero(void* dst, const void* src, bool there) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
-               "l"(src), "r"(there ? 16 : 0));
-}
-
 // ROWS rows of A by 64 rows of W; thread (ty, tx): rows ty * TM .. + TM - 1, columns tx + 16 j.
 template <int ROWS, int STAGES>
 __global__ void __launch_bounds__(kTileThreads)
@@ -138,7 +134,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
       const int g = of_a ? m0 + r : n0 + r - ROWS;
       const bool there = k < k_hi && g < (of_a ? M : N);
       const float* src = of_a ? A + (there ? g * lda + k : 0) : W + (there ? g * ldw + k : 0);
-      copy_16_or_zero(dst + r * kTileLd + piece, src, there);
+      mma::copy_async_16_or_zero(dst + r * kTileLd + piece, src, there);
     }
   };
   // the weights are written by no kernel: their first tiles are on the way while the kernel before this one ends

@@ -35,6 +35,7 @@
 //
 // States, decays, gates and sums are 32-bit whatever the storage type T.  The decay is applied as S + (a - 1) S with a - 1
 // formed by expm1, so that a state that remembers long keeps the distance of its decay from one.
+#include "chunks.cuh"
 #include "common.cuh"
 #include "mma.cuh"
 
@@ -231,33 +232,7 @@ memory_recurrence_kernel(const MemoryArgs p) {
 }
 
 // ---- by chunks of 64 rows ---------------------------------------------------------------------------------------------
-constexpr int kChunkRows = 64;
-
-struct ChunkPlace { int request, first, rows, index; };      // rows first .. first + rows - 1 of the step; index: of the step
-
-// The x-th chunk of the step's requests that have more than small_rows rows (request -1: there is none).
-__device__ __forceinline__ ChunkPlace find_chunk(const MemoryArgs& p, int x) {
-  ChunkPlace c = {-1, 0, 0, x};
-  int t = x;
-  for (int r = 0; r < p.requests; ++r) {
-    const int lo = p.cu_q[r], n = p.cu_q[r + 1] - lo;
-    if (n <= p.small_rows || p.state_slots[r] < 0) continue;
-    const int chunks = (n + kChunkRows - 1) / kChunkRows;
-    if (t < chunks) {
-      c.request = r;
-      c.first = lo + t * kChunkRows;
-      c.rows = min(kChunkRows, n - t * kChunkRows);
-      break;
-    }
-    t -= chunks;
-  }
-  return c;
-}
-__device__ __forceinline__ ChunkPlace find_chunk_shared(const MemoryArgs& p, int x, ChunkPlace* place) {
-  if (threadIdx.x == 0) *place = find_chunk(p, x);
-  __syncthreads();
-  return *place;
-}
+constexpr int kChunkRows = chunks::kRows;
 
 __device__ __forceinline__ float warp_scan_sum(float v, int lane) {
 #pragma unroll
@@ -364,10 +339,10 @@ memory_gates_kernel(const MemoryArgs p) {
 // kChannel: a thread a (chunk, channel), the chunk's rows in order.
 __global__ void __launch_bounds__(128)
 memory_channels_kernel(const MemoryArgs p) {
-  __shared__ ChunkPlace place;
+  __shared__ chunks::Place place;
   wait_for_prior_kernels();
   launch_dependents();
-  const ChunkPlace c = find_chunk_shared(p, blockIdx.x, &place);
+  const chunks::Place c = chunks::find(p.cu_q, p.state_slots, p.requests, p.small_rows, blockIdx.x, &place);
   if (c.request < 0) return;
   const int at = blockIdx.y * 128 + threadIdx.x, channels = p.heads * p.dim;
   if (at >= channels) return;
@@ -427,10 +402,10 @@ memory_chunk_state_kernel(const MemoryArgs p) {
   bf16* kh = reinterpret_cast<bf16*>(chunk_state_smem);      // [64 rows][kKeyLd]: scaled keys, rounded; the remainders
   bf16* kl = kh + kChunkRows * kKeyLd;
   bf16* vs = kl + kChunkRows * kKeyLd;                       // [64 rows][VT + 8]
-  __shared__ ChunkPlace place;
+  __shared__ chunks::Place place;
   wait_for_prior_kernels();
   launch_dependents();
-  const ChunkPlace c = find_chunk_shared(p, blockIdx.x, &place);
+  const chunks::Place c = chunks::find(p.cu_q, p.state_slots, p.requests, p.small_rows, blockIdx.x, &place);
   if (c.request < 0) return;
   const int h = blockIdx.y, vtiles = (p.vdim + VT - 1) / VT;
   const int d0 = static_cast<int>(blockIdx.z) / vtiles * kTileDim, v0 = static_cast<int>(blockIdx.z) % vtiles * VT;
@@ -531,7 +506,7 @@ memory_chunk_state_kernel(const MemoryArgs p) {
     }
   }
   const int da = d0 + warp * 16 + (lane >> 2), db = da + 8;
-  float* base = p.chunk_states + (static_cast<long long>(c.index) * p.heads + h) * p.dim * p.ld_state;
+  float* base = p.chunk_states + (static_cast<long long>(blockIdx.x) * p.heads + h) * p.dim * p.ld_state;
 #pragma unroll
   for (int i = 0; i < VT / 8; ++i) {
     const int col = v0 + i * 8 + 2 * (lane & 3);
@@ -555,14 +530,7 @@ memory_state_pass_kernel(const MemoryArgs p) {
   const int r = blockIdx.x, h = blockIdx.y;
   const int lo = p.cu_q[r], n = p.cu_q[r + 1] - lo, slot = p.state_slots[r];
   if (n <= p.small_rows || slot < 0) return;
-  if (threadIdx.x == 0) {
-    int at = 0;
-    for (int o = 0; o < r; ++o) {
-      const int m = p.cu_q[o + 1] - p.cu_q[o];
-      if (m > p.small_rows && p.state_slots[o] >= 0) at += (m + kChunkRows - 1) / kChunkRows;
-    }
-    first_chunk = at;
-  }
+  if (threadIdx.x == 0) first_chunk = chunks::first_of(p.cu_q, p.state_slots, p.small_rows, r);
   __syncthreads();
   const int pieces = p.vdim / 4 + (GATE == kExp ? 1 : 0);
   const int at = blockIdx.z * 128 + threadIdx.x;
@@ -650,11 +618,11 @@ memory_chunk_out_kernel(const MemoryArgs p) {
   bf16* sl = sh + kTileDim * (VT + 8);                       // ... and remainders
   bf16* vs = sl + kTileDim * (VT + 8);                       // [64 rows][VT + 8]
   float* Ls = reinterpret_cast<float*>(vs + kChunkRows * (VT + 8));   // kChannel: [64 rows][kDecayLd]
-  __shared__ ChunkPlace place;
+  __shared__ chunks::Place place;
   __shared__ float L_s[kChunkRows], w_s[kChunkRows];         // kStep, kExp
   wait_for_prior_kernels();
   launch_dependents();
-  const ChunkPlace c = find_chunk_shared(p, blockIdx.x, &place);
+  const chunks::Place c = chunks::find(p.cu_q, p.state_slots, p.requests, p.small_rows, blockIdx.x, &place);
   if (c.request < 0) return;
   const int h = blockIdx.y, v0 = static_cast<int>(blockIdx.z) * VT, g = h / p.per_group;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, quad = lane & 3;
@@ -667,7 +635,7 @@ memory_chunk_out_kernel(const MemoryArgs p) {
     L_s[tid] = p.log_decay[item];
     w_s[tid] = p.strength[item];
   }
-  const float* state = p.chunk_states + (static_cast<long long>(c.index) * p.heads + h) * p.dim * p.ld_state;
+  const float* state = p.chunk_states + (static_cast<long long>(blockIdx.x) * p.heads + h) * p.dim * p.ld_state;
   float O[VT / 8][4], P[8][4], N[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
   for (int i = 0; i < VT / 8; ++i) O[i][0] = O[i][1] = O[i][2] = O[i][3] = 0.0f;

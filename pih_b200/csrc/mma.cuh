@@ -12,6 +12,11 @@ __device__ __forceinline__ void copy_async_16(void* smem, const void* gmem) {
   const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
 }
+// (zeros where there is nothing; ``gmem`` is a readable address all the same)
+__device__ __forceinline__ void copy_async_16_or_zero(void* smem, const void* gmem, bool there) {
+  const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(there ? 16 : 0));
+}
 __device__ __forceinline__ void copy_async_4(void* smem, const void* gmem) {
   const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem));

@@ -263,12 +263,12 @@ retention_chunk_state_kernel(const RetentionArgs p) {
   if (c.request < 0) return;
   const int h = blockIdx.y, v0 = blockIdx.z * VT, tid = threadIdx.x;
   chunks::load_rows<DIM, DIM>(ks, p.k + (static_cast<long long>(c.first) * p.heads + h) * DIM, static_cast<long long>(p.heads) * DIM, c.rows);
-  chunks::copies_commit();
+  mma::copy_async_commit();
   if (tid < chunks::kRows) power[tid] = decay_power(log1pf(p.decay_m1[h]), max(0, c.rows - 1 - tid));
   chunks::load_rows<VT, VT>(vs, p.v + c.first * p.ldv + static_cast<long long>(h) * p.vdim + v0, p.ldv, c.rows);
   __syncthreads();
   for (int e = tid; e < chunks::kRows * VT; e += 256) vs[e] *= power[e / VT];
-  chunks::copies_wait();
+  mma::copy_async_wait<0>();
   __syncthreads();
   constexpr int RM = DIM / 16, RN = VT / 16;
   float2 U[RM][RN / 2];
@@ -351,9 +351,9 @@ retention_chunk_out_kernel(const RetentionArgs p) {
   const long long at = (static_cast<long long>(c.first) * p.heads + h) * DIM, ld = static_cast<long long>(p.heads) * DIM;
   chunks::load_rows<DIM, LD>(qs, p.q + at, ld, c.rows);
   chunks::load_rows<DIM, LD>(ks, p.k + at, ld, c.rows);
-  chunks::copies_commit();
+  mma::copy_async_commit();
   if (tid <= chunks::kRows) power[tid] = decay_power(log1pf(p.decay_m1[h]), tid);
-  chunks::copies_wait();
+  mma::copy_async_wait<0>();
   __syncthreads();
   {
     float2 s[4][4];
@@ -375,8 +375,8 @@ retention_chunk_out_kernel(const RetentionArgs p) {
   for (int d0 = 0; d0 < DIM; d0 += chunks::kRows) {
     __syncthreads();                                       // (what lay there is done with)
     chunks::load_rows<VT, VT>(ks, state + static_cast<long long>(d0) * p.vdim, p.vdim, chunks::kRows);
-    chunks::copies_commit();
-    chunks::copies_wait();
+    mma::copy_async_commit();
+    mma::copy_async_wait<0>();
     __syncthreads();
     chunks::multiply_columns<4, RN>(o, qs + d0, LD, ks, VT, chunks::kRows);
   }

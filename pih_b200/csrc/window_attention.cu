@@ -26,29 +26,11 @@
 //                            32-bit; the weights enter the product with the values as a bf16 pair (rounding and remainder)
 #include "common.cuh"
 #include "mma.cuh"
+#include "window_rule.cuh"
 
 namespace pih {
 
 constexpr int kWinMaxPerLane = 16;          // value columns a lane at most: vdim <= 512 (instances: 2, 4, 8, 16)
-
-// What a row may see, and how a score is finished: shared by all kernels of the file.
-struct WindowRule {
-  int window;            // 0: every earlier key
-  int chunk;             // 0: none; only keys of the row's own chunk of this many places
-  int keep_first;        // keys below this place stay seen
-  float scale;
-  float cap;             // 0: scores are not capped
-  const float* bias;     // [heads][distances] or null
-  int distances;
-  float out_scale;       // multiplies the output
-  int gate_columns;      // columns of the gate a head: 0: one number a head, else vdim of them
-  // the first key that a row at ``pos`` sees (apart from the kept ones); grows with ``pos``
-  __device__ __forceinline__ int first_of(int pos) const {
-    int first = window > 0 ? max(0, pos - window + 1) : 0;
-    if (chunk > 0 && pos > 0) first = max(first, pos - pos % chunk);
-    return first;
-  }
-};
 
 template <bool kExact>
 __device__ __forceinline__ float capped(float s, float cap) {
@@ -887,6 +869,12 @@ static int launch_window_tile(cudaStream_t s, unsigned tiles, const void* q, voi
   return 0;
 }
 
+extern "C" int pih_window_attention_tcgen05(const void* q, void* out, long long ldo, const void* cache, const void* block_table,
+                                            int table_width, const void* cu_q, const void* q_start, int rows, int requests,
+                                            int heads, int kv_heads, int dim, int vdim, int page_size, int num_pages,
+                                            const WindowRule* rule, const void* sink, const void* gate, long long ld_gate,
+                                            int small_rows, void* error, void* stream);
+
 // 1 when the tensor-core kernel has an instance for these sizes (bf16; dim and vdim multiples of 8 up to 128).
 extern "C" int pih_window_attention_tile_takes(int dim, int vdim) {
   return dim >= 8 && vdim >= 8 && dim % 8 == 0 && vdim % 8 == 0 && dim <= 128 && vdim <= 128;
@@ -924,11 +912,14 @@ extern "C" int pih_window_attention(int dtype, const void* q, void* out, long lo
   const int small_rows = tile ? 16 : 0x7fffffff;
   if (tile) {
     const unsigned tiles = static_cast<unsigned>((rows + kTileRows - 1) / kTileRows + requests);
-    int rc;
+    int rc = pih_window_attention_tcgen05(q, out, ldo, cache, block_table, table_width, cu_q, q_start, rows, requests, heads, kv_heads,
+                                          dim, vdim, page_size, num_pages, &rule, sink, gate, ld_gate, small_rows, error, stream);
+    if (rc != 0 && rc != PIH_ERR_UNSUPPORTED) return rc;
 #define PIH_TILE(D, V)                                                                                                 \
   rc = launch_window_tile<D, V>(s, tiles, q, out, ldo, cache, block_table, table_width, cu_q, q_start, requests, heads,    \
                                 kv_heads, dim, vdim, page_size, num_pages, rule, sink, gate, ld_gate, small_rows, error)
-    if (dim <= 32) { if (vdim <= 64) PIH_TILE(32, 64); else PIH_TILE(32, 128); }
+    if (rc == 0) {}
+    else if (dim <= 32) { if (vdim <= 64) PIH_TILE(32, 64); else PIH_TILE(32, 128); }
     else if (dim <= 64) { if (vdim <= 64) PIH_TILE(64, 64); else PIH_TILE(64, 128); }
     else { if (vdim <= 64) PIH_TILE(128, 64); else PIH_TILE(128, 128); }
 #undef PIH_TILE

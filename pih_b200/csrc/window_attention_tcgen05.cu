@@ -1,0 +1,397 @@
+// Window attention of prompts (window_attention.cu) on the 5th-generation tensor cores: keys and values of 64 or 128
+// columns, no cap and no bias by distance.  Same formula; the weights enter the product with the values as a bf16 pair
+// (rounding and remainder), as they do there.
+//
+// Bound by the special-function unit and the issue of the softmax (64 exponentials a row and tile: by count about 650 cycles
+// for 128 rows) beside 770 cycles of products; on mma.sync (128 rows, 8 warps, 64 keys) the operands' way from shared memory to
+// registers alone, once for each of the eight warps, took as long.  So
+//   a block is 128 rows of a (request, head), a tile 64 keys: S [128 x 64], the weights' roundings and remainders (32 columns
+//     each) and O [128 x VDIM] fill 256 columns of tensor memory and 96 KB of shared memory, and two blocks share an SM: one's
+//     products run under the other's softmax;
+//   warps 0-3  softmax, a thread a row: its 64 scores by one tcgen05.ld, no exchange between lanes.  O is multiplied only when
+//              a row's maximum has grown by more than 2^8 (the reference that stays is the one that the sum is formed with);
+//   warps 4-5  keys and values, a warp each, by cp.async into the 128-byte swizzle, two buffers each; places in the cache are
+//              looked up by row, so every page size is taken;
+//   warp 6     a thread issues S = Q K^T of the next tile as soon as this one's scores have been read, then O += P V.
+// A weight of zero times an infinite or NaN value that the row does not see would be NaN: a row whose sums are not finite
+// is computed again by its thread alone, over the keys that it sees.
+//
+// 2048 rows of 16 heads over a window of 1024 keys: 130 us on mma.sync, 48 here; 1531 rows of 8 heads in chunks of 1024: 85 and
+// 37 (96 blocks: an SM each, so the chain of a tile, and not the units, bounds it).
+#include "mma.cuh"
+#include "tcgen05.cuh"
+#include "window_rule.cuh"
+
+namespace pih {
+
+constexpr int kWuRows = 128, kWuKeys = 64, kWuThreads = 224;
+constexpr float kWuLog2e = 1.4426950408889634f;
+constexpr float kWuGrowth = 8.0f;                           // log2 of what a maximum may grow by before O is multiplied
+constexpr uint32_t kWuP = 64, kWuO = 128, kWuColumns = 256;  // tensor memory: S at 0, P (roundings, remainders), O
+
+template <int DIM, int VDIM>
+struct WindowUmmaSmem {
+  alignas(1024) unsigned char q[DIM / 64][kWuRows * 128];
+  alignas(1024) unsigned char k[2][DIM / 64][kWuKeys * 128];
+  alignas(1024) unsigned char v[2][VDIM / 64][kWuKeys * 128];
+  alignas(8) uint64_t q_full, k_full[2], v_full[2], s_full, s_read, p_full, o_done;
+  int tile_info[2];
+  uint32_t tmem_base;
+};
+
+struct WindowUmmaArgs {
+  const __nv_bfloat16* q;
+  __nv_bfloat16* out;
+  long long ldo;
+  const __nv_bfloat16* cache;
+  const int* block_table;
+  int table_width;
+  const int* cu_q;
+  const int* q_start;
+  int requests, heads, kv_heads, page_size, num_pages;
+  WindowRule rule;
+  const float* sink;
+  const __nv_bfloat16* gate;
+  long long ld_gate;
+  int small_rows;
+  uint32_t* error;
+};
+
+template <int DIM, int VDIM>
+__global__ void __launch_bounds__(kWuThreads, 2) window_attention_umma_kernel(const WindowUmmaArgs p) {
+  typedef __nv_bfloat16 bf16;
+  typedef WindowUmmaSmem<DIM, VDIM> Smem;
+  constexpr int KP = DIM / 64, VP = VDIM / 64;
+  extern __shared__ unsigned char smem_raw[];
+  Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const WindowRule& rule = p.rule;
+  wait_for_prior_kernels();
+  launch_dependents();
+  if (tid == 0) {
+    // the last tiles of a request have the most keys: they start first, so that the short ones fill the end
+    int t = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x), found = -1, at = 0;
+    for (int r = 0; r < p.requests; ++r) {
+      const int n = p.cu_q[r + 1] - p.cu_q[r];
+      if (n <= p.small_rows) continue;
+      const int tiles = (n + kWuRows - 1) / kWuRows;
+      if (t < tiles) { found = r; at = p.cu_q[r] + t * kWuRows; break; }
+      t -= tiles;
+    }
+    sm.tile_info[0] = found;
+    sm.tile_info[1] = at;
+    mbar_init(&sm.q_full, 4);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&sm.k_full[b], 1);
+      mbar_init(&sm.v_full[b], 1);
+    }
+    mbar_init(&sm.s_full, 1);
+    mbar_init(&sm.s_read, 4);
+    mbar_init(&sm.p_full, 4);
+    mbar_init(&sm.o_done, 1);
+    mbar_init_fence();
+  }
+  __syncthreads();
+  const int req = sm.tile_info[0];
+  if (req < 0) return;
+  if (warp == 6) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&sm.tmem_base)),
+                 "r"(kWuColumns));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = sm.tmem_base;
+  const int row0 = sm.tile_info[1];
+  const int nrows = min(kWuRows, p.cu_q[req + 1] - row0);
+  const int pos0 = p.q_start[req] + (row0 - p.cu_q[req]);
+  const int head = blockIdx.y, g = head / (p.heads / p.kv_heads);
+  const long long width = static_cast<long long>(p.kv_heads) * (DIM + VDIM);
+  const int* table = p.block_table + static_cast<long long>(req) * p.table_width;
+  const int key_last = pos0 + nrows - 1;
+  const int key_first = rule.first_of(pos0);
+  const int kept = min(rule.keep_first, key_first);          // kept keys that lie before the first row's first key
+  // the tiles in the order they are visited: those of the kept keys that end before the window's first tile, then the window's
+  const int tile_lo = key_first >> 6, tile_hi = key_last >> 6;
+  const int kept_tiles = kept > 0 ? min(((kept - 1) >> 6) + 1, tile_lo) : 0;
+  const int visits = kept_tiles + (tile_hi - tile_lo + 1);
+  auto tile_of = [&](int v) { return v < kept_tiles ? v : tile_lo + (v - kept_tiles); };
+  // the slot of the cache that holds key j, -1: none
+  auto slot_of = [&](int j) {
+    const int page = table[j / p.page_size];
+    if (page < 0 || page >= p.num_pages) {
+      publish_error(p.error, kRowWithoutPage);
+      return -1;
+    }
+    return page * p.page_size + j % p.page_size;
+  };
+
+  if (warp == 4 || warp == 5) {
+    // ---- warp 4 keys, warp 5 values: eight lanes 128 bytes of a row, rows (lane >> 3) + 4 i
+    const bool keys = warp == 4;
+    const int piece = lane & 7, r0 = lane >> 3;
+    const bf16* from = p.cache + (keys ? static_cast<long long>(g) * DIM : static_cast<long long>(p.kv_heads) * DIM + static_cast<long long>(g) * VDIM) + piece * 8;
+    auto fetch = [&](int v) {
+      const int j0 = tile_of(v) * kWuKeys;
+      int slots[2];                                          // of keys lane and lane + 32
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int j = j0 + lane + 32 * i;
+        slots[i] = j <= key_last && (j >= key_first || j < kept) ? slot_of(j) : -1;
+      }
+      unsigned char* to = keys ? sm.k[v & 1][0] : sm.v[v & 1][0];
+#pragma unroll
+      for (int i = 0; i < kWuKeys / 4; ++i) {
+        const int key = r0 + 4 * i, slot = __shfl_sync(0xffffffffu, slots[i >> 3], key & 31);
+        const bf16* src = from + (slot >= 0 ? slot * width : 0);
+        unsigned char* dst = to + key * 128 + ((piece ^ (key & 7)) << 4);
+#pragma unroll
+        for (int s = 0; s < (KP > VP ? KP : VP); ++s)
+          if (s < (keys ? KP : VP)) mma::copy_async_16_or_zero(dst + s * kWuKeys * 128, src + s * 64, slot >= 0);
+      }
+      mma::copy_async_commit();
+    };
+    // A key buffer is free when the scores of its tile are there, a value buffer when the products with its tile are done: a
+    // tile's copies are under way for the time of a whole tile.
+    fetch(0);
+    if (visits > 1) fetch(1);
+    for (int v = 0; v < visits; ++v) {
+      if (v + 1 < visits) mma::copy_async_wait<1>();
+      else mma::copy_async_wait<0>();
+      proxy_fence();                                         // this thread's copies of tile v are there, for the tensor cores too
+      __syncwarp();
+      if (lane == 0) mbar_arrive(keys ? &sm.k_full[v & 1] : &sm.v_full[v & 1]);
+      if (v + 2 < visits) {
+        if (!__all_sync(0xffffffffu, mbar_wait(keys ? &sm.s_full : &sm.o_done, v & 1, p.error))) break;
+        fetch(v + 2);
+      }
+    }
+    mma::copy_async_wait<0>();
+  } else if (warp == 6) {
+    // ---- products
+    if (lane == 0) {
+      constexpr uint32_t idesc_s = idesc_bf16(kWuRows, kWuKeys, false), idesc_o = idesc_bf16(kWuRows, VDIM, true);
+      auto scores = [&](int v) {
+        if (!mbar_wait(&sm.k_full[v & 1], (v >> 1) & 1, p.error)) return false;
+        tc_fence_after();
+#pragma unroll
+        for (int kk = 0; kk < DIM / 16; ++kk)
+          umma(tmem, desc_kmajor(smem_u32(sm.q[kk / 4]) + (kk % 4) * 32), desc_kmajor(smem_u32(sm.k[v & 1][kk / 4]) + (kk % 4) * 32),
+               idesc_s, kk > 0 ? 1u : 0u);
+        umma_commit(&sm.s_full);
+        return true;
+      };
+      bool alive = mbar_wait(&sm.q_full, 0, p.error) && scores(0);
+      for (int v = 0; v < visits && alive; ++v) {
+        if (v + 1 < visits) alive = mbar_wait(&sm.s_read, v & 1, p.error) && scores(v + 1);
+        if (!alive || !mbar_wait(&sm.p_full, v & 1, p.error) || !mbar_wait(&sm.v_full[v & 1], (v >> 1) & 1, p.error)) break;
+        tc_fence_after();
+        const uint64_t vd = desc_mnmajor(smem_u32(sm.v[v & 1][0]), kWuKeys * 128);
+#pragma unroll
+        for (int part = 0; part < 2; ++part)                 // the roundings, then the remainders
+#pragma unroll
+          for (int kk = 0; kk < kWuKeys / 16; ++kk)
+            umma_a_tmem(tmem + kWuO, tmem + kWuP + part * 32 + kk * 8, vd + ((kk * 16 * 128) >> 4), idesc_o,
+                        (v > 0 || part > 0 || kk > 0) ? 1u : 0u);
+        umma_commit(&sm.o_done);
+      }
+    }
+  } else {
+    // ---- softmax: a thread a row
+    for (int rr = tid >> 3; rr < kWuRows; rr += 16) {        // the rows' queries, on their way as the keys are
+      const bool there = rr < nrows;
+      const bf16* src = p.q + (static_cast<long long>(row0 + (there ? rr : 0)) * p.heads + head) * DIM + (tid & 7) * 8;
+#pragma unroll
+      for (int s = 0; s < KP; ++s)
+        mma::copy_async_16_or_zero(sm.q[s] + rr * 128 + (((tid & 7) ^ (rr & 7)) << 4), src + s * 64, there);
+    }
+    mma::copy_async_commit();
+    mma::copy_async_wait<0>();
+    proxy_fence();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sm.q_full);
+    const uint32_t lanes = tmem + (static_cast<uint32_t>(warp * 32) << 16);
+    const int row = warp * 32 + lane;
+    const int pos = row < nrows ? pos0 + row : -1, first = rule.first_of(pos);
+    const int warp_first = pos0 + warp * 32, first_high = rule.first_of(min(warp_first + 31, key_last));
+    const float c = rule.scale * kWuLog2e;
+    float m = -INFINITY, l = 0.0f;
+    bool alive = true;
+    for (int v = 0; v < visits; ++v) {
+      alive = mbar_wait(&sm.s_full, v & 1, p.error);
+      if (!__all_sync(0xffffffffu, alive)) { alive = false; break; }
+      tc_fence_after();
+      uint32_t s[64];
+      tmem_ld64(lanes, s);
+      tmem_wait_ld();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.s_read);
+      const int j0 = tile_of(v) * kWuKeys;
+      // a tile that every row of the warp sees whole needs no mask
+      const bool whole = j0 + 63 <= warp_first && (j0 >= first_high || j0 + 63 < rule.keep_first);
+      float top = -INFINITY;
+      if (!whole) {
+#pragma unroll
+        for (int i = 0; i < 64; ++i) {
+          const int key = j0 + i;
+          const bool seen = key <= pos && (key >= first || key < rule.keep_first);
+          if (!seen) s[i] = 0xff800000u;
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 64; ++i) top = fmaxf(top, __uint_as_float(s[i]));
+      top *= c;                                              // (c > 0)
+      const bool grown = top > m + kWuGrowth || (m == -INFINITY && top > -INFINITY);
+      const float fix = grown ? mma::exp2_fast(m - top) : 1.0f;
+      if (grown) m = top;
+      const float ref = m == -INFINITY ? 0.0f : m;
+      float sum0 = 0.0f, sum1 = 0.0f;
+      uint32_t w[64];                                        // roundings in pairs, then remainders
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const float a = mma::exp2_fast(fmaf(__uint_as_float(s[2 * i]), c, -ref)), b = mma::exp2_fast(fmaf(__uint_as_float(s[2 * i + 1]), c, -ref));
+        sum0 += a;
+        sum1 += b;
+        w[i] = mma::pack(a, b);
+        w[32 + i] = mma::pack_remainder(a, b, w[i]);
+      }
+      l = fmaf(l, fix, sum0 + sum1);
+      if (v > 0) {                                           // the product before has read P and added to O
+        alive = mbar_wait(&sm.o_done, (v - 1) & 1, p.error);
+        if (!__all_sync(0xffffffffu, alive)) { alive = false; break; }
+        tc_fence_after();
+        if (__any_sync(0xffffffffu, fix != 1.0f)) {
+#pragma unroll 1
+          for (int n = 0; n < VDIM; n += 16) {
+            uint32_t o[16];
+            tmem_ld16(lanes + kWuO + n, o);
+            tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * fix);
+            tmem_st16(lanes + kWuO + n, o);
+          }
+        }
+      }
+      tmem_st64(lanes + kWuP, w);
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.p_full);
+    }
+    alive = alive && mbar_wait(&sm.o_done, (visits - 1) & 1, p.error);
+    __syncwarp();
+    tc_fence_after();
+    float fold = 1.0f, total = l;
+    if (p.sink != nullptr) {                                 // the sink's term, in the exp2 domain like the others
+      const float s = p.sink[head] * kWuLog2e, high = fmaxf(m, s);
+      fold = exp2f(m - high);
+      total = fmaf(l, fold, exp2f(s - high));
+    }
+    if (row < nrows && alive && (!(total > 0.0f) || total > 3.0e38f)) publish_error(p.error, kAttentionDenominator);
+    float f = total > 0.0f ? fold / total * rule.out_scale : 0.0f;
+    const bf16* gate = p.gate == nullptr || row >= nrows ? nullptr : p.gate + (row0 + row) * p.ld_gate + static_cast<long long>(head) * max(rule.gate_columns, 1);
+    if (gate != nullptr && rule.gate_columns == 0) f *= 1.0f / (1.0f + __expf(-__bfloat162float(gate[0])));
+    bf16* dst = p.out + static_cast<long long>(row0 + row) * p.ldo + static_cast<long long>(head) * VDIM;
+#pragma unroll 1
+    for (int n = 0; n < VDIM; n += 32) {
+      uint32_t o[32];
+      tmem_ld32(lanes + kWuO + n, o);
+      tmem_wait_ld();
+      if (row >= nrows) continue;                            // (the loads above are the whole warp's)
+      bool finite = true;
+#pragma unroll
+      for (int i = 0; i < 32; ++i) finite = finite && (o[i] & 0x7f800000u) != 0x7f800000u;
+      if (!finite) {
+        const bf16* qr = p.q + (static_cast<long long>(row0 + row) * p.heads + head) * DIM;
+        float acc[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
+        for (int j = 0; j <= pos; ++j) {
+          if (j < first && j >= rule.keep_first) { j = first - 1; continue; }
+          const int slot = slot_of(j);
+          if (slot < 0) continue;
+          const long long at = slot * width;
+          const bf16* kr = p.cache + at + static_cast<long long>(g) * DIM;
+          const bf16* vr = p.cache + at + static_cast<long long>(p.kv_heads) * DIM + static_cast<long long>(g) * VDIM + n;
+          float dot = 0.0f;
+          for (int i = 0; i < DIM; ++i) dot = fmaf(__bfloat162float(qr[i]), __bfloat162float(kr[i]), dot);
+          const float weight = mma::exp2_fast(fmaf(dot, c, m == -INFINITY ? 0.0f : -m));
+#pragma unroll
+          for (int i = 0; i < 32; ++i) acc[i] = fmaf(weight, __bfloat162float(vr[i]), acc[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(acc[i]);
+      }
+#pragma unroll
+      for (int i = 0; i < 32; i += 8) {
+        uint32_t packed[4];
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) {
+          float a = __uint_as_float(o[i + e]), b = __uint_as_float(o[i + e + 1]);
+          if (gate != nullptr && rule.gate_columns > 0) {
+            a *= __fdividef(1.0f, 1.0f + __expf(-__bfloat162float(gate[n + i + e])));
+            b *= __fdividef(1.0f, 1.0f + __expf(-__bfloat162float(gate[n + i + e + 1])));
+          }
+          packed[e / 2] = mma::pack(a * f, b * f);
+        }
+        *reinterpret_cast<uint4*>(dst + n + i) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+      }
+    }
+    tc_fence_before();
+  }
+  __syncwarp();
+  __syncthreads();
+  if (warp == 6) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kWuColumns));
+}
+
+template <int DIM, int VDIM>
+static int launch_window_umma(const WindowUmmaArgs& p, unsigned tiles, cudaStream_t s) {
+  const int smem = static_cast<int>(sizeof(WindowUmmaSmem<DIM, VDIM>)) + 1024;
+  static bool raised = false;                               // per instance
+  if (!raised) {
+    const cudaError_t e = cudaFuncSetAttribute(window_attention_umma_kernel<DIM, VDIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    raised = true;
+  }
+  launch_kernel(window_attention_umma_kernel<DIM, VDIM>, dim3(tiles, p.heads), dim3(kWuThreads), smem, s, p);
+  PIH_LAUNCH_CHECK();
+  return 0;
+}
+
+}  // namespace pih
+
+using namespace pih;
+
+// The rows of requests of more than small_rows rows, bf16.  PIH_ERR_UNSUPPORTED where the other kernel has to do it: sizes
+// other than 64 and 128, a cap, a bias, a scale that is not positive, rows of q, cache or output that do not begin on 16 bytes.
+extern "C" int pih_window_attention_tcgen05(const void* q, void* out, long long ldo, const void* cache, const void* block_table,
+                                            int table_width, const void* cu_q, const void* q_start, int rows, int requests,
+                                            int heads, int kv_heads, int dim, int vdim, int page_size, int num_pages,
+                                            const WindowRule* rule, const void* sink, const void* gate, long long ld_gate,
+                                            int small_rows, void* error, void* stream) {
+  if ((dim != 64 && dim != 128) || (vdim != 64 && vdim != 128) || rule->cap > 0.0f || rule->bias != nullptr || !(rule->scale > 0.0f) ||
+      ldo % 8 || ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(cache)) & 15))
+    return PIH_ERR_UNSUPPORTED;
+  WindowUmmaArgs p = {};
+  p.q = static_cast<const __nv_bfloat16*>(q);
+  p.out = static_cast<__nv_bfloat16*>(out);
+  p.ldo = ldo;
+  p.cache = static_cast<const __nv_bfloat16*>(cache);
+  p.block_table = static_cast<const int*>(block_table);
+  p.table_width = table_width;
+  p.cu_q = static_cast<const int*>(cu_q);
+  p.q_start = static_cast<const int*>(q_start);
+  p.requests = requests, p.heads = heads, p.kv_heads = kv_heads, p.page_size = page_size, p.num_pages = num_pages;
+  p.rule = *rule;
+  p.sink = static_cast<const float*>(sink);
+  p.gate = static_cast<const __nv_bfloat16*>(gate);
+  p.ld_gate = ld_gate;
+  p.small_rows = small_rows;
+  p.error = static_cast<uint32_t*>(error);
+  const unsigned tiles = static_cast<unsigned>((rows + kWuRows - 1) / kWuRows + requests);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (dim == 64) return vdim == 64 ? launch_window_umma<64, 64>(p, tiles, s) : launch_window_umma<64, 128>(p, tiles, s);
+  return vdim == 64 ? launch_window_umma<128, 64>(p, tiles, s) : launch_window_umma<128, 128>(p, tiles, s);
+}

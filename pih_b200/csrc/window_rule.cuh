@@ -1,0 +1,27 @@
+// What the kernels of the window attention share.
+#pragma once
+
+#include "common.cuh"
+
+namespace pih {
+
+// What a row may see, and how a score is finished: shared by all kernels of the file.
+struct WindowRule {
+  int window;            // 0: every earlier key
+  int chunk;             // 0: none; only keys of the row's own chunk of this many places
+  int keep_first;        // keys below this place stay seen
+  float scale;
+  float cap;             // 0: scores are not capped
+  const float* bias;     // [heads][distances] or null
+  int distances;
+  float out_scale;       // multiplies the output
+  int gate_columns;      // columns of the gate a head: 0: one number a head, else vdim of them
+  // the first key that a row at ``pos`` sees (apart from the kept ones); grows with ``pos``
+  __device__ __forceinline__ int first_of(int pos) const {
+    int first = window > 0 ? max(0, pos - window + 1) : 0;
+    if (chunk > 0 && pos > 0) first = max(first, pos - pos % chunk);
+    return first;
+  }
+};
+
+}  // namespace pih

@@ -109,6 +109,27 @@ __device__ __forceinline__ float warp_min(float v) {
   return v;
 }
 
+// v[0 .. COUNT-1]: a lane's shares of COUNT rows.  Afterwards v[0 .. max(1, COUNT / 2^steps)-1] are whole sums (over the lanes
+// that differ in the bits of MASK and below) of the rows from the returned one on.
+template <int COUNT, int MASK>
+__device__ __forceinline__ int fold_shares(float* v, int part) {
+  if constexpr (MASK == 0) {
+    return 0;
+  } else if constexpr (COUNT == 1) {
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], MASK);
+    return fold_shares<1, MASK / 2>(v, part);
+  } else {
+    constexpr int H = COUNT / 2;
+    const bool upper = (part & MASK) != 0;
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+      const float send = upper ? v[i] : v[i + H], keep = upper ? v[i + H] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, MASK);
+    }
+    return (upper ? H : 0) + fold_shares<H, MASK / 2>(v, part);
+  }
+}
+
 // Sum over a block of up to 1024 threads; every thread gets the result.  The
 // order of additions depends only on blockDim, never on other rows or blocks.
 __device__ __forceinline__ float block_sum(float v, float* scratch /* >= 33 floats */) {

@@ -46,52 +46,36 @@ struct ScanArgs {
   int inner, states;
 };
 
-// v[0 .. COUNT-1]: a lane's shares of COUNT rows.  Afterwards v[0 .. max(1, COUNT / 2^steps)-1] are whole sums (over the lanes
-// that differ in the bits of MASK and below) of the rows from the returned one on.
-template <int COUNT, int MASK>
-__device__ __forceinline__ int fold_shares(float* v, int part) {
-  if constexpr (MASK == 0) {
-    return 0;
-  } else if constexpr (COUNT == 1) {
-    v[0] += __shfl_xor_sync(0xffffffffu, v[0], MASK);
-    return fold_shares<1, MASK / 2>(v, part);
-  } else {
-    constexpr int H = COUNT / 2;
-    const bool upper = (part & MASK) != 0;
-#pragma unroll
-    for (int i = 0; i < H; ++i) {
-      const float send = upper ? v[i] : v[i + H], keep = upper ? v[i + H] : v[i];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, MASK);
-    }
-    return (upper ? H : 0) + fold_shares<H, MASK / 2>(v, part);
-  }
-}
-
 template <int kParts>
 struct ScanShape {
   static constexpr int CH = kParts >= 4 ? 16 : 64 / kParts;            // channels a block
   static constexpr int kThreads = CH * kParts;
 };
 
-template <typename T, int kParts, int kN>
-__global__ void __launch_bounds__(ScanShape<kParts>::kThreads)
+// kAhead: the block has twice the threads; the first half runs (2) of chunk i while the second half runs (3) of chunk i - 1
+// and (1) of chunk i + 1, with one barrier a chunk instead of two.  Otherwise every thread does all three in turn, each waiting
+// for the other's latencies: 1531 rows of 2048 channels with 16 states, 128 blocks of four warps, 85 us so, 66 with the halves.
+template <typename T, int kParts, int kN, bool kAhead>
+__global__ void __launch_bounds__(ScanShape<kParts>::kThreads * (kAhead ? 2 : 1))
 selective_scan_kernel(const ScanArgs p) {
   constexpr bool kExact = sizeof(T) == 4;
   constexpr int CH = ScanShape<kParts>::CH, TH = ScanShape<kParts>::kThreads;
   constexpr int NP = kParts * kN;                                       // states with the padding
   constexpr int E = (kScanRows * CH + TH - 1) / TH;                     // (row, channel) pairs a thread
   constexpr int EB = kScanRows * 2 * NP / TH;                           // numbers of B and C a thread
+  constexpr int kBuffer = kScanRows * (2 * NP + 3 * CH);                // words of a chunk
   static_assert(kScanRows * 2 * NP % TH == 0 && kN % 2 == 0, "whole shares, 8-byte loads");
   extern __shared__ __align__(16) float scan_smem[];
   typedef float2 (*Steps)[CH];
   typedef float (*Vectors)[2][NP];
   typedef float (*Outputs)[CH];
-  Vectors bc_s = reinterpret_cast<Vectors>(scan_smem);                  // [rows][B, C][NP]
-  Steps steps = reinterpret_cast<Steps>(scan_smem + kScanRows * 2 * NP);                    // [rows][CH]: (dt, dt x)
-  Outputs y_s = reinterpret_cast<Outputs>(scan_smem + kScanRows * (2 * NP + 2 * CH));       // [rows][CH]
+  auto bc_of = [&](int b) { return reinterpret_cast<Vectors>(scan_smem + b * kBuffer); };                                  // [rows][B, C][NP]
+  auto steps_of = [&](int b) { return reinterpret_cast<Steps>(scan_smem + b * kBuffer + kScanRows * 2 * NP); };            // [rows][CH]: (dt, dt x)
+  auto y_of = [&](int b) { return reinterpret_cast<Outputs>(scan_smem + b * kBuffer + kScanRows * (2 * NP + 2 * CH)); };   // [rows][CH]
   wait_for_prior_kernels();
   launch_dependents();
-  const int r = blockIdx.x, c0 = blockIdx.y * CH, tid = threadIdx.x;
+  const int r = blockIdx.x, c0 = blockIdx.y * CH, tid = threadIdx.x % TH;
+  const bool scans = !kAhead || threadIdx.x < TH, helps = !kAhead || threadIdx.x >= TH;
   const int lo = p.cu_q[r], hi = p.cu_q[r + 1], slot = p.state_slots[r];
   if (hi <= lo || slot < 0) return;
   const T* u = static_cast<const T*>(p.u);
@@ -102,19 +86,21 @@ selective_scan_kernel(const ScanArgs p) {
   const bool live = c < p.inner;
   float* Sg = p.state + slot * p.state_stride + static_cast<long long>(c) * p.states;
   float S[kN], A[kN];
+  if (scans) {
 #pragma unroll
-  for (int i = 0; i < kN; ++i) {
-    const bool there = live && n0 + i < p.states;
-    S[i] = there ? Sg[n0 + i] : 0.0f;
-    A[i] = there ? p.A[static_cast<long long>(c) * p.states + n0 + i] * (kExact ? 1.0f : 1.4426950408889634f) : 0.0f;
+    for (int i = 0; i < kN; ++i) {
+      const bool there = live && n0 + i < p.states;
+      S[i] = there ? Sg[n0 + i] : 0.0f;
+      A[i] = there ? p.A[static_cast<long long>(c) * p.states + n0 + i] * (kExact ? 1.0f : 1.4426950408889634f) : 0.0f;
+    }
   }
   // pair e of this thread: row (tid + e TH) / CH of the chunk, channel (tid + e TH) % CH of the block
   float bias[E], skip[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) {
     const int ce = c0 + (tid + e * TH) % CH;
-    bias[e] = ce < p.inner ? p.dt_bias[ce] : 0.0f;
-    skip[e] = ce < p.inner ? p.D[ce] : 0.0f;
+    bias[e] = helps && ce < p.inner ? p.dt_bias[ce] : 0.0f;
+    skip[e] = helps && ce < p.inner ? p.D[ce] : 0.0f;
   }
   // the next chunk's numbers, as they lie in memory: nothing is computed from them before they are needed
   T nx[E], nz[E], nbc[EB];
@@ -135,23 +121,26 @@ selective_scan_kernel(const ScanArgs p) {
       nbc[e] = t < hi && n < p.states ? bc[t * p.ldbc + which * p.states + n] : zero;
     }
   };
-  fetch(lo);
-  for (int t0 = lo; t0 < hi; t0 += kScanRows) {
-    const int n_rows = min(kScanRows, hi - t0);
-    float x[E];
-    T zz[E];
+  // (1), from what has been fetched
+  struct Held { T x[E], z[E]; };
+  auto prepare = [&](int b, Held& held) {
+    Steps steps = steps_of(b);
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       const int idx = tid + e * TH;
-      x[e] = to_float<T>(nx[e]);
-      zz[e] = nz[e];
+      held.x[e] = nx[e];
+      held.z[e] = nz[e];
       const float dt = softplus_f(nt[e] + bias[e]);
-      if (idx < kScanRows * CH) steps[idx / CH][idx % CH] = make_float2(dt, dt * x[e]);
+      if (idx < kScanRows * CH) steps[idx / CH][idx % CH] = make_float2(dt, dt * to_float<T>(nx[e]));
     }
 #pragma unroll
-    for (int e = 0; e < EB; ++e) scan_smem[tid + e * TH] = to_float<T>(nbc[e]);
-    __syncthreads();
-    if (t0 + kScanRows < hi) fetch(t0 + kScanRows);
+    for (int e = 0; e < EB; ++e) scan_smem[b * kBuffer + tid + e * TH] = to_float<T>(nbc[e]);
+  };
+  // (2)
+  auto scan = [&](int b, int n_rows) {
+    Vectors bc_s = bc_of(b);
+    Steps steps = steps_of(b);
+    Outputs y_s = y_of(b);
     float share[kScanRows];
     auto row = [&](int t) {
       const float2 st = steps[t][cl];
@@ -186,51 +175,107 @@ selective_scan_kernel(const ScanArgs p) {
     constexpr int kKept = kScanRows / kParts > 0 ? kScanRows / kParts : 1;
 #pragma unroll
     for (int i = 0; i < kKept; ++i) y_s[first + i][cl] = share[i];      // (more lanes than rows: two write the same sum)
-    __syncthreads();
+  };
+  // (3)
+  auto finish = [&](int b, int t0, const Held& held) {
+    Outputs y_s = y_of(b);
+    const int n_rows = min(kScanRows, hi - t0);
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       const int idx = tid + e * TH, t = idx / CH, ce = c0 + idx % CH;
       if (idx < kScanRows * CH && t < n_rows && ce < p.inner) {
-        const float y = fmaf(skip[e], x[e], y_s[t][idx % CH]);
-        out[(t0 + t) * p.ldo + ce] = from_float<T>(silu_times<T>(to_float<T>(zz[e]), y) * p.out_scale);
+        const float y = fmaf(skip[e], to_float<T>(held.x[e]), y_s[t][idx % CH]);
+        out[(t0 + t) * p.ldo + ce] = from_float<T>(silu_times<T>(to_float<T>(held.z[e]), y) * p.out_scale);
       }
     }
-    // (y_s is written again only behind the next chunk's first barrier, steps and bc_s only behind this chunk's second)
+  };
+  if constexpr (!kAhead) {
+    Held held;
+    fetch(lo);
+    for (int t0 = lo; t0 < hi; t0 += kScanRows) {
+      prepare(0, held);
+      __syncthreads();
+      if (t0 + kScanRows < hi) fetch(t0 + kScanRows);
+      scan(0, min(kScanRows, hi - t0));
+      __syncthreads();
+      finish(0, t0, held);
+      // (y_s is written again only behind the next chunk's first barrier, steps and bc_s only behind this chunk's second)
+    }
+  } else {
+    // buffer b: chunk i with i % 2 == b.  Behind the barrier of chunk i - 1 its steps, B and C are free (chunk i + 1 goes
+    // there), its sums are whole, and chunk i's steps, B and C are there.
+    Held before, held, next;                                            // of chunks i - 1, i and i + 1
+    if (helps) {
+      fetch(lo);
+      prepare(0, held);
+      fetch(lo + kScanRows);
+    }
+    __syncthreads();
+    int b = 0;
+    for (int t0 = lo; t0 < hi; t0 += kScanRows, b ^= 1) {
+      if (scans) {
+        scan(b, min(kScanRows, hi - t0));
+      } else {
+        if (t0 + kScanRows < hi) {
+          prepare(b ^ 1, next);
+          fetch(t0 + 2 * kScanRows);
+        }
+        if (t0 > lo) finish(b ^ 1, t0 - kScanRows, before);
+        before = held;
+        held = next;
+      }
+      __syncthreads();
+    }
+    if (helps) finish(b ^ 1, lo + (hi - lo - 1) / kScanRows * kScanRows, before);
   }
-  if (live) {
+  if (scans && live) {
 #pragma unroll
     for (int i = 0; i < kN; ++i)
       if (n0 + i < p.states) Sg[n0 + i] = S[i];
   }
 }
 
-template <typename T, int kParts, int kN>
-static void launch_scan(const ScanArgs& p, int requests, cudaStream_t s) {
+template <typename T, int kParts, int kN, bool kAhead>
+static void launch_scan_as(const ScanArgs& p, const dim3& grid, bool alone, cudaStream_t s) {
   constexpr int CH = ScanShape<kParts>::CH;
-  const dim3 grid(requests, (p.inner + CH - 1) / CH);
-  const int needed = kScanRows * (2 * kParts * kN + 3 * CH) * static_cast<int>(sizeof(float));
-  // the rows follow one another: with no more blocks than SMs every block asks for more than half of an SM's shared memory
-  // and so gets an SM alone
-  const bool alone = static_cast<long long>(grid.x) * grid.y <= 148;
+  const int needed = kScanRows * (2 * kParts * kN + 3 * CH) * (kAhead ? 2 : 1) * static_cast<int>(sizeof(float));
   const int smem = alone && needed < 116 * 1024 ? 116 * 1024 : needed;
   static int raised = 48 * 1024;                               // (per instance)
   if (smem > raised) {
-    cudaFuncSetAttribute(selective_scan_kernel<T, kParts, kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaFuncSetAttribute(selective_scan_kernel<T, kParts, kN, kAhead>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     raised = smem;
   }
-  launch_kernel(selective_scan_kernel<T, kParts, kN>, grid, dim3(ScanShape<kParts>::kThreads), smem, s, p);
+  launch_kernel(selective_scan_kernel<T, kParts, kN, kAhead>, grid, dim3(ScanShape<kParts>::kThreads * (kAhead ? 2 : 1)), smem, s, p);
+}
+
+template <typename T, int kParts, int kN>
+static void launch_scan(const ScanArgs& p, int rows, int requests, cudaStream_t s) {
+  constexpr int CH = ScanShape<kParts>::CH;
+  const dim3 grid(requests, (p.inner + CH - 1) / CH);
+  // the rows follow one another: with no more blocks than SMs every block asks for more than half of an SM's shared memory
+  // and so gets an SM alone
+  const long long blocks = static_cast<long long>(grid.x) * grid.y;
+  const bool alone = blocks <= 148;
+  // twice the threads a block where there is more than a chunk to overlap and the SMs have room for them
+  if constexpr (kParts <= 16) {
+    if (blocks <= 2 * 148 && rows > 2 * kScanRows) {
+      launch_scan_as<T, kParts, kN, true>(p, grid, alone, s);
+      return;
+    }
+  }
+  launch_scan_as<T, kParts, kN, false>(p, grid, alone, s);
 }
 
 template <typename T>
-static int dispatch_scan(const ScanArgs& p, int requests, cudaStream_t s) {
+static int dispatch_scan(const ScanArgs& p, int rows, int requests, cudaStream_t s) {
   const int n = p.states;
-  if (n <= 4) launch_scan<T, 2, 2>(p, requests, s);
-  else if (n <= 8) launch_scan<T, 4, 2>(p, requests, s);
-  else if (n <= 16) launch_scan<T, 8, 2>(p, requests, s);
-  else if (n <= 32) launch_scan<T, 16, 2>(p, requests, s);
-  else if (n <= 64) launch_scan<T, 32, 2>(p, requests, s);
-  else if (n <= 128) launch_scan<T, 32, 4>(p, requests, s);
-  else if (n <= 256) launch_scan<T, 32, 8>(p, requests, s);
+  if (n <= 4) launch_scan<T, 2, 2>(p, rows, requests, s);
+  else if (n <= 8) launch_scan<T, 4, 2>(p, rows, requests, s);
+  else if (n <= 16) launch_scan<T, 8, 2>(p, rows, requests, s);
+  else if (n <= 32) launch_scan<T, 16, 2>(p, rows, requests, s);
+  else if (n <= 64) launch_scan<T, 32, 2>(p, rows, requests, s);
+  else if (n <= 128) launch_scan<T, 32, 4>(p, rows, requests, s);
+  else if (n <= 256) launch_scan<T, 32, 8>(p, rows, requests, s);
   else return PIH_ERR_UNSUPPORTED;
   PIH_LAUNCH_CHECK();
   return 0;
@@ -263,7 +308,7 @@ extern "C" int pih_selective_scan(int dtype, const void* u, long long ldu, const
   p.state_slots = static_cast<const int*>(state_slots);
   p.inner = inner, p.states = states;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (dtype == PIH_F32) return dispatch_scan<float>(p, requests, s);
-  if (dtype == PIH_BF16) return dispatch_scan<__nv_bfloat16>(p, requests, s);
+  if (dtype == PIH_F32) return dispatch_scan<float>(p, rows, requests, s);
+  if (dtype == PIH_BF16) return dispatch_scan<__nv_bfloat16>(p, rows, requests, s);
   return PIH_ERR_BAD_ARGUMENT;
 }

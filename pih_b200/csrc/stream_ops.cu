@@ -46,6 +46,86 @@ stream_norm_add_kernel(float* __restrict__ h, const TY* __restrict__ y, long lon
   }
 }
 
+// The same for rows whose pieces of eight lie on 16 bytes: a thread keeps up to kHeld pieces of y and h, all asked for before
+// the row's sum, so that a row costs one trip to memory instead of two and the stream's second reading (2048 rows of 1024:
+// 10.1 us by the element-wise form above, 5.5 by this one, 3.7 for the bytes).
+template <typename T>
+__device__ __forceinline__ void load_eight(float (&v)[8], const T* src) {
+  if constexpr (sizeof(T) == 2) {
+    const uint4 r = *reinterpret_cast<const uint4*>(src);
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&r);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = __bfloat1622float2(h[i]);
+      v[2 * i] = f.x, v[2 * i + 1] = f.y;
+    }
+  } else {
+    const float4 a = reinterpret_cast<const float4*>(src)[0], b = reinterpret_cast<const float4*>(src)[1];
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+  }
+}
+template <typename T>
+__device__ __forceinline__ void store_eight(T* dst, const float (&v)[8]) {
+  if constexpr (sizeof(T) == 2) {
+    uint4 r;
+    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&r);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+    *reinterpret_cast<uint4*>(dst) = r;
+  } else {
+    reinterpret_cast<float4*>(dst)[0] = make_float4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<float4*>(dst)[1] = make_float4(v[4], v[5], v[6], v[7]);
+  }
+}
+
+template <typename TY, typename TO, int kHeld>
+__global__ void __launch_bounds__(512)
+stream_norm_add_pieces_kernel(float* __restrict__ h, const TY* __restrict__ y, long long ldy, const float* __restrict__ bias,
+                              const float* __restrict__ weight, TO* __restrict__ copy, int width, float eps) {
+  __shared__ float scratch[33];
+  wait_for_prior_kernels();
+  launch_dependents();
+  const long long row = blockIdx.x;
+  const TY* yr = y + row * ldy;
+  float* hr = h + row * width;
+  float v[kHeld][8], s[kHeld][8];
+#pragma unroll
+  for (int u = 0; u < kHeld; ++u) {
+    const int c = 8 * (threadIdx.x + u * blockDim.x);
+    if (c < width) {
+      load_eight<TY>(v[u], yr + c);
+      load_eight<float>(s[u], hr + c);
+    }
+  }
+  float ss = 0.0f;
+#pragma unroll
+  for (int u = 0; u < kHeld; ++u) {
+    const int c = 8 * (threadIdx.x + u * blockDim.x);
+    if (c >= width) continue;
+    if (bias != nullptr) {
+      float b[8];
+      load_eight<float>(b, bias + c);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[u][i] += b[i];
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ss = fmaf(v[u][i], v[u][i], ss);
+  }
+  ss = block_sum(ss, scratch);
+  const float inv = 1.0f / sqrtf(ss / static_cast<float>(width) + eps);
+#pragma unroll
+  for (int u = 0; u < kHeld; ++u) {
+    const int c = 8 * (threadIdx.x + u * blockDim.x);
+    if (c >= width) continue;
+    float w[8];
+    load_eight<float>(w, weight + c);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s[u][i] += v[u][i] * inv * w[i];
+    store_eight<float>(hr + c, s[u]);
+    if (copy != nullptr) store_eight<TO>(copy + row * width + c, s[u]);
+  }
+}
+
 template <typename T>
 __global__ void bias_xielu_kernel(const T* __restrict__ z, long long ldz, const float* __restrict__ bias, T* __restrict__ out,
                                   long long rows, int width, float alpha_positive, float alpha_negative) {
@@ -260,15 +340,27 @@ extern "C" int pih_stream_norm_add(int y_dtype, int copy_dtype, void* h, const v
   if (rows <= 0) return 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const dim3 grid(rows), block(width >= 1024 ? 256 : 128);
+  const int threads = (width + 7) / 8;                       // of a piece each
+  const bool pieces = width % 8 == 0 && ldy % 8 == 0 && threads <= 1024 &&
+                      ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(bias) |
+                        reinterpret_cast<uintptr_t>(weight) | reinterpret_cast<uintptr_t>(copy)) & 15) == 0;
+  const dim3 few((threads <= 512 ? threads + 31 : (threads + 1) / 2 + 31) / 32 * 32);
+#define PIH_SNA_AS(KERNEL, BLOCK, TY, TO)                                                                              \
+  launch_kernel(KERNEL, grid, BLOCK, 0, s, static_cast<float*>(h), static_cast<const TY*>(y), ldy,                     \
+                static_cast<const float*>(bias), static_cast<const float*>(weight), static_cast<TO*>(copy), width, eps)
 #define PIH_SNA(TY, TO)                                                                                                \
-  launch_kernel(stream_norm_add_kernel<TY, TO>, grid, block, 0, s, static_cast<float*>(h), static_cast<const TY*>(y), \
-                ldy, static_cast<const float*>(bias), static_cast<const float*>(weight), static_cast<TO*>(copy), width, eps)
+  do {                                                                                                                 \
+    if (!pieces) PIH_SNA_AS((stream_norm_add_kernel<TY, TO>), block, TY, TO);                                          \
+    else if (threads <= 512) PIH_SNA_AS((stream_norm_add_pieces_kernel<TY, TO, 1>), few, TY, TO);                      \
+    else PIH_SNA_AS((stream_norm_add_pieces_kernel<TY, TO, 2>), few, TY, TO);                                          \
+  } while (0)
   if (y_dtype == PIH_BF16 && copy_dtype == PIH_BF16) PIH_SNA(bf16, bf16);
   else if (y_dtype == PIH_F32 && copy_dtype == PIH_F32) PIH_SNA(float, float);
   else if (y_dtype == PIH_BF16 && copy_dtype == PIH_F32) PIH_SNA(bf16, float);
   else if (y_dtype == PIH_F32 && copy_dtype == PIH_BF16) PIH_SNA(float, bf16);
   else return PIH_ERR_BAD_ARGUMENT;
 #undef PIH_SNA
+#undef PIH_SNA_AS
   PIH_LAUNCH_CHECK();
   return 0;
 }

@@ -544,6 +544,81 @@ latent_merge_kernel(const float* __restrict__ partial, const T* __restrict__ gat
   }
 }
 
+// The same, bit for bit, with a warp a (row, head), for the few parts of a prompt: nothing meets in a block, and the loads of a
+// row's columns (pairs) run beside those of the other seven warps.  2048 rows of 8 heads of rank 256 in two parts: a block
+// each took 35 us behind the attention, most of it one warp's chain of loads and exponentials while seven waited; this, 8.
+constexpr int kFewParts = 4;
+
+template <typename T>
+__global__ void __launch_bounds__(256)
+latent_merge_rows_kernel(const float* __restrict__ partial, const T* __restrict__ gate, long long ldg,
+                         const float* __restrict__ sink, const int* __restrict__ request_of_row, T* __restrict__ out,
+                         long long items, int heads, int rank, int splits, uint32_t* err) {
+  wait_for_prior_kernels();
+  launch_dependents();
+  const long long item = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (item >= items) return;
+  const int row = static_cast<int>(item / heads), h = static_cast<int>(item % heads);
+  if (request_of_row[row] < 0) return;
+  const float* base = partial + item * splits * (rank + 2);
+  constexpr int kAhead = 4;                                  // pairs of columns a lane: ranks up to 256 in one round
+  float2 v[2][kAhead];
+  auto load = [&](int s, int c0, float2 (&to)[kAhead]) {
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int c = c0 + 2 * (lane + 32 * u);
+      if (c < rank) to[u] = *reinterpret_cast<const float2*>(base + s * (rank + 2) + 2 + c);
+    }
+  };
+  load(0, 0, v[0]);
+  if (splits > 1) load(1, 0, v[1]);
+  float m = -INFINITY, ls = 0.0f;
+  if (lane < splits) {
+    m = base[lane * (rank + 2)];
+    ls = base[lane * (rank + 2) + 1];
+  }
+  float m_all = sink != nullptr ? sink[h] : -INFINITY;
+  if (ls > 0.0f) m_all = fmaxf(m_all, m);
+  m_all = warp_max(m_all);
+  const float factor = ls > 0.0f ? expf(m - m_all) : 0.0f;
+  float l = warp_sum(fmaf(ls, factor, 0.0f));
+  if (sink != nullptr) l += expf(sink[h] - m_all);
+  if (!(l > 0.0f) || !isfinite(l)) {
+    if (lane == 0) publish_error(err, kAttentionDenominator);
+    l = 1.0f;
+  }
+  float scale_out = 1.0f / l;
+  if (gate != nullptr) {
+    const float z = to_float<T>(gate[static_cast<long long>(row) * ldg + h]);
+    scale_out *= 1.0f / (1.0f + expf(-z));
+  }
+  for (int c0 = 0; c0 < rank; c0 += 64 * kAhead) {
+    float2 a[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) a[u] = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int s = 0; s < kFewParts; ++s) {
+      if (s >= splits) break;
+      if (c0 > 0 || s > 1) load(s, c0, v[s & 1]);
+      const float f = __shfl_sync(0xffffffffu, factor, s);
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const float2 x = v[s & 1][u];
+        a[u].x = fmaf(x.x, f, a[u].x);
+        a[u].y = fmaf(x.y, f, a[u].y);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int c = c0 + 2 * (lane + 32 * u);
+      if (c >= rank) continue;
+      out[item * rank + c] = from_float<T>(a[u].x * scale_out);
+      out[item * rank + c + 1] = from_float<T>(a[u].y * scale_out);
+    }
+  }
+}
+
 }  // namespace pih
 
 using namespace pih;
@@ -712,10 +787,19 @@ extern "C" int pih_latent_attention_mma(const void* q, const void* gate, long lo
 #undef PIH_LM
 #undef PIH_LM1
   PIH_LAUNCH_CHECK();
+  const int parts = splits * (rows_per_block == 1 ? 8 : 2);
+  if (parts <= kFewParts && items >= 8 * 148) {                       // (fewer: a block each fills the SMs no less)
+    launch_kernel(latent_merge_rows_kernel<bf16>, dim3(static_cast<unsigned>((items + 7) / 8)), dim3(256), 0, s,
+                  static_cast<const float*>(partial), static_cast<const bf16*>(gate), ldg, static_cast<const float*>(sink),
+                  static_cast<const int*>(request_of_row), static_cast<bf16*>(out), items, heads, rank, parts,
+                  static_cast<uint32_t*>(err));
+    PIH_LAUNCH_CHECK();
+    return 0;
+  }
   launch_kernel(latent_merge_kernel<bf16>, dim3(static_cast<unsigned>(items)), dim3(rank >= 256 ? 256 : (rank + 31) / 32 * 32), 0, s,
                 static_cast<const float*>(partial), static_cast<const bf16*>(gate), ldg, static_cast<const float*>(sink),
                 static_cast<const int*>(request_of_row), static_cast<bf16*>(out), rows, heads, rank,
-                splits * (rows_per_block == 1 ? 8 : 2), static_cast<uint32_t*>(err));
+                parts, static_cast<uint32_t*>(err));
   PIH_LAUNCH_CHECK();
   return 0;
 }

@@ -707,8 +707,11 @@ class CudaOps:
                 out = self.gate_mul(out.view(T, B * N), gate, "sigmoid").view(T, B, N)
             return out
         if x.dtype == torch.bfloat16 and out_dtype == torch.bfloat16 and T >= self.batched_library_min_rows:
-            # many rows in bf16: the library's batched product (32-bit accumulation), as the single products of many rows
-            return torch.bmm(x.transpose(0, 1), w.transpose(1, 2)).transpose(0, 1).contiguous()
+            # many rows in bf16: the library's batched product (32-bit accumulation), as the single products of many rows,
+            # written where it belongs (a product by heads and a copy into rows took 8 us more for 2048 x 8 x 256)
+            out = torch.empty(T, B, N, dtype=out_dtype, device=x.device)
+            torch.bmm(x.transpose(0, 1), w.transpose(1, 2), out=out.transpose(0, 1))
+            return out
         out = torch.empty(T, B, N, dtype=out_dtype, device=x.device)
         if x.dtype == torch.bfloat16 and T <= self.skinny_max_rows and K % 8 == 0:
             # few rows in bf16: a warp an output column, the small matrices' rows streamed once

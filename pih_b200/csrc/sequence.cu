@@ -563,12 +563,12 @@ __global__ void delta_recurrence_kernel(const float* __restrict__ qn, const floa
 }
 
 // The same recurrence with S in registers, for the key sizes that have an instance.  Block (request, head, 16 value
-// columns); a column of S is held by 8 threads (4 for small keys, 16 for 256), thread (column c = tid / parts, part p = tid %
+// columns); a column of S is held by 8 threads (4 for small keys, 16 for 256 and in blocks of 8), thread (column c = tid / parts, part p = tid %
 // parts) every parts-th piece of four rows from piece p on: the parts of a column sit in neighbouring lanes, meet through
 // shuffles, and read neighbouring 16-byte pieces of k and q (no bank conflicts).
 //
 // What a token costs is the chain from its state to the next one's, so both products that read the state are taken from the
-// SAME (decayed) state g S and meet in the same shuffles: with a = (g S)^T k and b = (g S)^T q,
+// SAME (decayed) state g S: with a = (g S)^T k and b = (g S)^T q,
 //     u = beta (v - a),    o = b + (k . q) u,    S <- g S + k u^T
 // — the read-out of the state after the write, without reading it again; k . q comes from delta_prepare.  Products and
 // updates take two numbers an instruction (fma.rn.f32x2: each half rounds as fma.rn.f32 does).
@@ -587,10 +587,16 @@ __device__ __forceinline__ void async_copy_4(void* smem_dst, const void* src) {
 __device__ __forceinline__ void async_copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void async_copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-template <int kDim, bool kChannel>
+// For keys of 64 and 128 there are two shapes, 16 columns by 8 parts and 8 columns by 16: the second halves what a thread
+// computes between two tokens and brings twice as many blocks, for the few columns of one request (1531 tokens, 8 heads of
+// 128 x 128: 325 us by 64 blocks of the first, 275 by 128 of the second).  Both add in the same order: a part of the first is parts p and p + 8 of the
+// second, each with sums of its own.
+template <int kDim, bool kChannel, int kColumns>
 struct DeltaShape {
-  static constexpr int kParts = kDim >= 256 ? 16 : (kDim >= 64 ? 8 : 4);   // threads a column of S
-  static constexpr int kCols = 16;                        // value columns a block
+  static constexpr bool kTwoShapes = kDim == 64 || kDim == 128;
+  static constexpr int kParts = kDim >= 256 || kColumns == 8 ? 16 : (kDim >= 64 ? 8 : 4);   // threads a column of S
+  static constexpr int kHalves = kTwoShapes && kColumns == 16 ? 2 : 1;     // sums a thread keeps apart
+  static constexpr int kCols = kColumns;                  // value columns a block
   static constexpr int kThreads = kCols * kParts;
   static constexpr int kRows = kDim / kParts;             // rows of S a thread holds
   static constexpr int kVecs = kChannel ? 3 : 2;          // vectors of kDim numbers staged a token: k | q (| decay - 1)
@@ -600,14 +606,14 @@ struct DeltaShape {
   static constexpr int words(int value_bytes) { return kTail + 4 + kCols * value_bytes / 4; }
 };
 
-template <typename T, int kDim, bool kChannel>
-__global__ void __launch_bounds__(DeltaShape<kDim, kChannel>::kThreads)
+template <typename T, int kDim, bool kChannel, int kColumns>
+__global__ void __launch_bounds__(DeltaShape<kDim, kChannel, kColumns>::kThreads)
 delta_recurrence_reg_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ qk_dot,
                             const T* __restrict__ v, long long ldv, const float* __restrict__ decay,
                             const float* __restrict__ beta, float* __restrict__ out, float* __restrict__ state,
                             long long state_stride, const int* __restrict__ cu_q, const int* __restrict__ state_slots,
                             int heads, int kv_heads, int vdim) {
-  typedef DeltaShape<kDim, kChannel> Shape;
+  typedef DeltaShape<kDim, kChannel, kColumns> Shape;
   constexpr int kParts = Shape::kParts, kThreads = Shape::kThreads, kRows = Shape::kRows;
   constexpr int kChunk = Shape::kChunk, kCols = Shape::kCols, kPairs = kRows / 2, kTail = Shape::kTail;
   constexpr int kVWords = kCols * sizeof(T) / 4;          // the block's values of a token, in 32-bit words
@@ -686,30 +692,40 @@ delta_recurrence_reg_kernel(const float* __restrict__ qn, const float* __restric
     x.kq = cur[kTail + 2];
     x.v = to_float<T>(reinterpret_cast<const T*>(cur + kTail + 4)[cl]);
   };
-  auto compute = [&](const Tok& x, int t) {
-    // two chains a product; the parts' sums of both products go through the shuffles side by side
-    float2 a0 = make_float2(0.0f, 0.0f), a1 = a0, b0 = a0, b1 = a0;
+  // The state's step.  Returns this lane's share of the read-out; the whole is the sum over the column's lanes, the pairs that
+  // differ in the highest bit first.
+  auto compute = [&](const Tok& x) -> float {
+    // Two chains a product and half.  What the next token waits for is a.
+    float2 a0[Shape::kHalves], a1[Shape::kHalves], b0[Shape::kHalves], b1[Shape::kHalves];
+#pragma unroll
+    for (int v = 0; v < Shape::kHalves; ++v) a0[v] = a1[v] = b0[v] = b1[v] = make_float2(0.0f, 0.0f);
 #pragma unroll
     for (int i = 0; i < kPairs; i += 2) {
+      const int v = (i >> 1) % Shape::kHalves;
       S[i] = fma2(x.g[kChannel ? i : 0], S[i], S[i]);            // g S, formed as S + (g - 1) S
       S[i + 1] = fma2(x.g[kChannel ? i + 1 : 0], S[i + 1], S[i + 1]);
-      a0 = fma2(S[i], x.k[i], a0);
-      a1 = fma2(S[i + 1], x.k[i + 1], a1);
-      b0 = fma2(S[i], x.q[i], b0);
-      b1 = fma2(S[i + 1], x.q[i + 1], b1);
+      a0[v] = fma2(S[i], x.k[i], a0[v]);
+      a1[v] = fma2(S[i + 1], x.k[i + 1], a1[v]);
     }
-    float a = (a0.x + a1.x) + (a0.y + a1.y), b = (b0.x + b1.x) + (b0.y + b1.y);
+    float a = (a0[0].x + a1[0].x) + (a0[0].y + a1[0].y);
+    if constexpr (Shape::kHalves == 2) a += (a0[1].x + a1[1].x) + (a0[1].y + a1[1].y);
+    if constexpr (Shape::kTwoShapes && kParts == 16) a += __shfl_xor_sync(0xffffffffu, a, 8);
 #pragma unroll
-    for (int m = 1; m < kParts; m <<= 1) {
-      const float pa = __shfl_xor_sync(0xffffffffu, a, m), pb = __shfl_xor_sync(0xffffffffu, b, m);
-      a += pa;
-      b += pb;
+    for (int m = 1; m < (Shape::kTwoShapes ? 8 : kParts); m <<= 1) a += __shfl_xor_sync(0xffffffffu, a, m);
+#pragma unroll
+    for (int i = 0; i < kPairs; i += 2) {
+      const int v = (i >> 1) % Shape::kHalves;
+      b0[v] = fma2(S[i], x.q[i], b0[v]);
+      b1[v] = fma2(S[i + 1], x.q[i + 1], b1[v]);
     }
     const float u = x.b * (x.v - a);
     const float2 uu = make_float2(u, u);
 #pragma unroll
     for (int i = 0; i < kPairs; ++i) S[i] = fma2(x.k[i], uu, S[i]);
-    if (live && part == 0) out[(static_cast<long long>(t) * heads + h) * vdim + col] = fmaf(x.kq, u, b);
+    float b = (b0[0].x + b1[0].x) + (b0[0].y + b1[0].y);
+    if (part == 0) b = fmaf(x.kq, u, b);
+    if constexpr (Shape::kHalves == 2) b += (b0[1].x + b1[1].x) + (b0[1].y + b1[1].y);
+    return b;
   };
   issue(lo, 0);
   async_copies_wait();
@@ -722,17 +738,28 @@ delta_recurrence_reg_kernel(const float* __restrict__ qn, const float* __restric
     Tok x0, x1;
     load(x0, base);
     if (n_tok == kChunk) {                                       // no branch a token: loads and sums of neighbours overlap
-#pragma unroll 2
+      // a lane's shares of the chunk's read-outs stay in registers and meet by halving exchanges, 15 shuffles for 16 tokens and
+      // 16 lanes instead of 64 on the way from token to token
+      float share[kChunk];
+#pragma unroll
       for (int tok = 0; tok < kChunk; tok += 2) {
         load(x1, base + (tok + 1) * kTok);
-        compute(x0, t0 + tok);
+        share[tok] = compute(x0);
         load(x0, base + min(tok + 2, kChunk - 1) * kTok);        // (the last one is not used)
-        compute(x1, t0 + tok + 1);
+        share[tok + 1] = compute(x1);
       }
+      const int first = fold_shares<kChunk, kParts / 2>(share, part);
+      constexpr int kKept = kChunk / kParts > 0 ? kChunk / kParts : 1;
+#pragma unroll
+      for (int i = 0; i < kKept; ++i)                            // (more lanes than tokens: two write the same sum)
+        if (live) out[(static_cast<long long>(t0 + first + i) * heads + h) * vdim + col] = share[i];
     } else {
       for (int tok = 0; tok < n_tok; ++tok) {
         load(x0, base + tok * kTok);
-        compute(x0, t0 + tok);
+        float o = compute(x0);
+#pragma unroll
+        for (int m = kParts / 2; m > 0; m >>= 1) o += __shfl_xor_sync(0xffffffffu, o, m);
+        if (live && part == 0) out[(static_cast<long long>(t0 + tok) * heads + h) * vdim + col] = o;
       }
     }
     async_copies_wait();
@@ -1043,11 +1070,11 @@ extern "C" int pih_causal_conv(int dtype, const void* x, long long ldx, const vo
 // key channel, with decay_bias of the same layout; decay_log [heads].  scratch: fp32, rows * (2 * kv_heads * dim + kv_heads +
 // heads + heads * (channels ? dim : 1)), 16-byte aligned.  out: fp32 [rows, heads, vdim].  The state S [heads, dim, vdim] lies at the
 // start of a request's slot.
-template <typename T, int D, bool CH>
-static void launch_delta_reg(cudaStream_t s, const float* qn, const float* kn, const float* qk_dot, const T* v, long long ld, const float* decay,
+template <typename T, int D, bool CH, int COLS>
+static void launch_delta_columns(cudaStream_t s, const float* qn, const float* kn, const float* qk_dot, const T* v, long long ld, const float* decay,
                              const float* beta, float* out, float* state, long long state_stride, const int* cu_q,
                              const int* state_slots, int requests, int heads, int kv_heads, int vdim) {
-  typedef DeltaShape<D, CH> Shape;
+  typedef DeltaShape<D, CH, COLS> Shape;
   const size_t needed = 2 * static_cast<size_t>(Shape::kChunk) * Shape::words(sizeof(T)) * sizeof(float);
   const dim3 grid(requests, heads, (vdim + Shape::kCols - 1) / Shape::kCols);
   // The chain from token to token is what a prompt costs: with no more blocks than SMs, every block asks for more than half
@@ -1056,12 +1083,28 @@ static void launch_delta_reg(cudaStream_t s, const float* qn, const float* kn, c
   const size_t staged = alone && needed < 116 * 1024 ? 116 * 1024 : needed;
   static size_t raised = 48 * 1024;                            // (per instance)
   if (staged > raised) {
-    cudaFuncSetAttribute(delta_recurrence_reg_kernel<T, D, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(delta_recurrence_reg_kernel<T, D, CH, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          static_cast<int>(staged));
     raised = staged;
   }
-  launch_kernel(delta_recurrence_reg_kernel<T, D, CH>, grid,
+  launch_kernel(delta_recurrence_reg_kernel<T, D, CH, COLS>, grid,
                 dim3(Shape::kThreads), staged, s, qn, kn, qk_dot, v, ld, decay, beta, out, state, state_stride, cu_q, state_slots, heads, kv_heads, vdim);
+}
+
+// Blocks of 16 columns, or of 8 where blocks of 16 leave half of the SMs without one.
+template <typename T, int D, bool CH>
+static void launch_delta_reg(cudaStream_t s, const float* qn, const float* kn, const float* qk_dot, const T* v, long long ld, const float* decay,
+                             const float* beta, float* out, float* state, long long state_stride, const int* cu_q,
+                             const int* state_slots, int requests, int heads, int kv_heads, int vdim) {
+  if constexpr (D == 64 || D == 128) {
+    if (static_cast<long long>(requests) * heads * ((vdim + 7) / 8) <= 148) {
+      launch_delta_columns<T, D, CH, 8>(s, qn, kn, qk_dot, v, ld, decay, beta, out, state, state_stride, cu_q, state_slots,
+                                        requests, heads, kv_heads, vdim);
+      return;
+    }
+  }
+  launch_delta_columns<T, D, CH, 16>(s, qn, kn, qk_dot, v, ld, decay, beta, out, state, state_stride, cu_q, state_slots, requests,
+                                     heads, kv_heads, vdim);
 }
 
 template <typename T, bool CH>

@@ -1,0 +1,365 @@
+// Attention over cached latents (latent_attention.cu) for prompts on the 5th-generation tensor cores: the heads of a token share
+// its keys and values, so a tile of 128 MMA rows is 128 / heads consecutive tokens of a request with all their heads, and one
+// copy of a tile of latents serves as the keys of S = Q L^T and as the values of O += P L.  Ranks of 64 to 256 in steps of 64,
+// head counts that divide 128.  Formula as there; the weights enter the product as a bf16 pair (rounding and remainder).
+//
+// On mma.sync the sums of 8 heads of rank 256 held most of a warp's registers, every warp fetched the tile's operands for its
+// own 16 rows, and the parts that eight warps left of a row were added up by another kernel.  Here
+//   a block is one tile of rows over all keys that it sees, 64 at a time; S (two), the pairs of weights (two, 64 columns) and O
+//     (up to 256) fill tensor memory; nothing is left to merge;
+//   warps 0-3  softmax, a thread a row; O is multiplied only when a maximum has grown by more than 2^8;
+//   warps 4-5  latents by cp.async into the 128-byte swizzle, three buffers; places are looked up by row (any page size);
+//   warp 6     a thread issues the scores of the next tile ahead of the products of this one.
+// By count a tile of rank 256 is 1540 cycles of products and 650 of softmax, which run side by side.
+//
+// A weight of zero times a latent that is not finite and not seen would be NaN: a row whose sums are not finite is computed
+// again by its thread alone, over the keys that it sees.  Waits are bounded.
+//
+// 2048 rows of 8 heads of rank 256 over a window of 1024: 149 us on mma.sync with its merge, 42 here (128 blocks, an SM each:
+// a tile takes 2.3 us, of which the products are 0.8; the chain of a tile bounds it).
+#include "mma.cuh"
+#include "tcgen05.cuh"
+
+namespace pih {
+
+constexpr int kLuRows = 128, kLuKeys = 64, kLuBuffers = 3, kLuThreads = 224;
+constexpr float kLuLog2e = 1.4426950408889634f;
+constexpr float kLuGrowth = 8.0f;                           // log2 of what a maximum may grow by before O is multiplied
+constexpr uint32_t kLuP = 128, kLuO = 256;                  // tensor memory: S at 0 and 64, P at 128 and 192, O
+
+template <int R>
+struct LatentUmmaSmem {
+  alignas(1024) unsigned char q[R / 64][kLuRows * 128];
+  alignas(1024) unsigned char tile[kLuBuffers][R / 64][kLuKeys * 128];
+  alignas(8) uint64_t q_full, full[kLuBuffers], s_full[2], s_read[2], p_full[2], o_done[2];
+  int tile_info[2];
+  uint32_t tmem_base;
+};
+
+struct LatentUmmaArgs {
+  const __nv_bfloat16* q;                                   // [rows, heads, R]
+  __nv_bfloat16* out;                                       // the same
+  const __nv_bfloat16* gate;                                // nullable, [rows, ld_gate], a logit a head
+  long long ld_gate;
+  const float* sink;                                        // nullable, [heads]
+  const __nv_bfloat16* cache;                               // [pages, page_size, R]
+  const int* block_table;
+  int table_width;
+  const int* positions;
+  const int* cu_q;
+  int requests, heads, page_size, num_pages, window;
+  float scale;
+  uint32_t* error;
+};
+
+template <int R>
+__global__ void __launch_bounds__(kLuThreads, 1) latent_attention_umma_kernel(const LatentUmmaArgs p) {
+  typedef __nv_bfloat16 bf16;
+  constexpr int PANELS = R / 64;
+  extern __shared__ unsigned char smem_raw[];
+  LatentUmmaSmem<R>& sm = *reinterpret_cast<LatentUmmaSmem<R>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tokens = kLuRows / p.heads;                      // of a tile
+  wait_for_prior_kernels();
+  launch_dependents();
+  if (tid == 0) {
+    // the last tiles of a request have the most keys: they start first, so that the short ones fill the end
+    int t = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x), found = -1, at = 0;
+    for (int r = 0; r < p.requests; ++r) {
+      const int tiles = (p.cu_q[r + 1] - p.cu_q[r] + tokens - 1) / tokens;
+      if (t < tiles) { found = r; at = p.cu_q[r] + t * tokens; break; }
+      t -= tiles;
+    }
+    sm.tile_info[0] = found;
+    sm.tile_info[1] = at;
+    mbar_init(&sm.q_full, 4);
+    for (int b = 0; b < kLuBuffers; ++b) mbar_init(&sm.full[b], 2);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&sm.s_full[b], 1);
+      mbar_init(&sm.s_read[b], 4);
+      mbar_init(&sm.p_full[b], 4);
+      mbar_init(&sm.o_done[b], 1);
+    }
+    mbar_init_fence();
+  }
+  __syncthreads();
+  const int req = sm.tile_info[0];
+  if (req < 0) return;
+  if (warp == 6) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&sm.tmem_base)), "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = sm.tmem_base;
+  const int row0 = sm.tile_info[1];
+  const int n_tokens = min(tokens, p.cu_q[req + 1] - row0);
+  const int nrows = n_tokens * p.heads, pos0 = p.positions[row0];
+  const bf16* q_tile = p.q + static_cast<long long>(row0) * p.heads * R;       // the tile's rows follow one another
+  const int* table = p.block_table + static_cast<long long>(req) * p.table_width;
+  auto first_of = [&](int pos) { return p.window > 0 ? max(0, pos - p.window + 1) : 0; };
+  const int key_last = pos0 + n_tokens - 1, key_first = first_of(pos0);
+  const int tile_lo = key_first >> 6, visits = (key_last >> 6) - tile_lo + 1;
+  // the slot of the cache that holds key j, -1: none
+  auto slot_of = [&](int j) {
+    const int page = table[j / p.page_size];
+    if (page < 0 || page >= p.num_pages) {
+      publish_error(p.error, kRowWithoutPage);
+      return -1;
+    }
+    return page * p.page_size + j % p.page_size;
+  };
+
+  if (warp == 4 || warp == 5) {
+    // ---- latents: a warp half of a tile's keys, eight lanes 128 bytes of a row, rows (lane >> 3) + 4 i of the half
+    const int piece = lane & 7, r0 = lane >> 3, half = (warp - 4) * 32;
+    auto fetch = [&](int v) {
+      const int j = (tile_lo + v) * kLuKeys + half + lane;
+      const int mine = j <= key_last && j >= key_first ? slot_of(j) : -1;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int slot = __shfl_sync(0xffffffffu, mine, r0 + 4 * i), key = half + r0 + 4 * i;
+        const bf16* src = p.cache + (slot >= 0 ? static_cast<long long>(slot) * R : 0) + piece * 8;
+        unsigned char* dst = sm.tile[v % kLuBuffers][0] + key * 128 + ((piece ^ (key & 7)) << 4);
+#pragma unroll
+        for (int s = 0; s < PANELS; ++s) mma::copy_async_16_or_zero(dst + s * kLuKeys * 128, src + s * 64, slot >= 0);
+      }
+      mma::copy_async_commit();
+    };
+    for (int v = 0; v < min(kLuBuffers, visits); ++v) fetch(v);
+    for (int v = 0; v < visits; ++v) {
+      // tiles asked for behind tile v: two before the first is handed over, then one
+      const int behind = min(visits, v == 0 ? kLuBuffers : v + 2) - (v + 1);
+      if (behind >= 2) mma::copy_async_wait<2>();
+      else if (behind == 1) mma::copy_async_wait<1>();
+      else mma::copy_async_wait<0>();
+      proxy_fence();                                         // this thread's copies of tile v are there, for the tensor cores too
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.full[v % kLuBuffers]);
+      // Tile v is handed over before the wait for the products of tile v - 1, whose buffer the next one takes: the scores of
+      // tile v are issued ahead of those products.
+      if (v >= 1 && v + 2 < visits) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&sm.o_done[(v - 1) & 1], ((v - 1) >> 1) & 1, p.error))) break;
+        fetch(v + 2);
+      }
+    }
+    mma::copy_async_wait<0>();
+  } else if (warp == 6) {
+    // ---- products
+    if (lane == 0) {
+      constexpr uint32_t idesc_s = idesc_bf16(kLuRows, kLuKeys, false), idesc_o = idesc_bf16(kLuRows, R, true);
+      auto scores = [&](int v) {
+        if (!mbar_wait(&sm.full[v % kLuBuffers], (v / kLuBuffers) & 1, p.error)) return false;
+        if (v >= 2 && !mbar_wait(&sm.s_read[v & 1], ((v - 2) >> 1) & 1, p.error)) return false;
+        tc_fence_after();
+        const uint32_t q_at = smem_u32(sm.q[0]), l_at = smem_u32(sm.tile[v % kLuBuffers][0]);
+#pragma unroll
+        for (int kk = 0; kk < R / 16; ++kk)
+          umma(tmem + (v & 1) * 64, desc_kmajor(q_at + (kk / 4) * kLuRows * 128 + (kk % 4) * 32),
+               desc_kmajor(l_at + (kk / 4) * kLuKeys * 128 + (kk % 4) * 32), idesc_s, kk > 0 ? 1u : 0u);
+        umma_commit(&sm.s_full[v & 1]);
+        return true;
+      };
+      bool alive = mbar_wait(&sm.q_full, 0, p.error) && scores(0);
+      for (int v = 0; v < visits && alive; ++v) {
+        if (v + 1 < visits) alive = scores(v + 1);
+        if (!alive || !mbar_wait(&sm.p_full[v & 1], (v >> 1) & 1, p.error)) break;
+        tc_fence_after();
+        const uint64_t ld = desc_mnmajor(smem_u32(sm.tile[v % kLuBuffers][0]), kLuKeys * 128);
+#pragma unroll
+        for (int part = 0; part < 2; ++part)                 // the roundings, then the remainders
+#pragma unroll
+          for (int kk = 0; kk < kLuKeys / 16; ++kk)
+            umma_a_tmem(tmem + kLuO, tmem + kLuP + (v & 1) * 64 + part * 32 + kk * 8, ld + ((kk * 16 * 128) >> 4), idesc_o,
+                        (v > 0 || part > 0 || kk > 0) ? 1u : 0u);
+        umma_commit(&sm.o_done[v & 1]);
+      }
+    }
+  } else {
+    // ---- softmax: a thread a row
+    for (int rr = tid >> 3; rr < kLuRows; rr += 16) {        // the rows' queries, on their way as the latents are
+      const bool there = rr < nrows;
+      const bf16* src = q_tile + (there ? rr : 0) * R + (tid & 7) * 8;
+#pragma unroll
+      for (int s = 0; s < PANELS; ++s)
+        mma::copy_async_16_or_zero(sm.q[s] + rr * 128 + (((tid & 7) ^ (rr & 7)) << 4), src + s * 64, there);
+    }
+    mma::copy_async_commit();
+    mma::copy_async_wait<0>();
+    proxy_fence();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sm.q_full);
+    const uint32_t lanes = tmem + (static_cast<uint32_t>(warp * 32) << 16);
+    const int row = warp * 32 + lane, head = row % p.heads;
+    const int pos = row < nrows ? pos0 + row / p.heads : -1, first = first_of(pos);
+    const int low = pos0 + warp * 32 / p.heads, high = first_of(min(pos0 + (warp * 32 + 31) / p.heads, key_last));   // of the warp's rows
+    const float c = p.scale * kLuLog2e;
+    float m = -INFINITY, l = 0.0f;
+    bool alive = true;
+    for (int v = 0; v < visits; ++v) {
+      alive = mbar_wait(&sm.s_full[v & 1], (v >> 1) & 1, p.error);
+      if (!__all_sync(0xffffffffu, alive)) { alive = false; break; }
+      tc_fence_after();
+      uint32_t s[64];
+      tmem_ld64(lanes + (v & 1) * 64, s);
+      tmem_wait_ld();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.s_read[v & 1]);
+      const int j0 = (tile_lo + v) * kLuKeys;
+      if (!(j0 + 63 <= low && j0 >= high)) {                 // (a tile that every row of the warp sees whole needs no mask)
+#pragma unroll
+        for (int i = 0; i < 64; ++i)
+          if (j0 + i > pos || j0 + i < first) s[i] = 0xff800000u;
+      }
+      float top = -INFINITY;
+#pragma unroll
+      for (int i = 0; i < 64; ++i) top = fmaxf(top, __uint_as_float(s[i]));
+      top *= c;                                              // (c > 0)
+      const bool grown = top > m + kLuGrowth || (m == -INFINITY && top > -INFINITY);
+      const float fix = grown ? mma::exp2_fast(m - top) : 1.0f;
+      if (grown) m = top;
+      const float ref = m == -INFINITY ? 0.0f : m;
+      float sum0 = 0.0f, sum1 = 0.0f;
+      uint32_t w[64];                                        // roundings in pairs, then remainders
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const float a = mma::exp2_fast(fmaf(__uint_as_float(s[2 * i]), c, -ref)), b = mma::exp2_fast(fmaf(__uint_as_float(s[2 * i + 1]), c, -ref));
+        sum0 += a;
+        sum1 += b;
+        w[i] = mma::pack(a, b);
+        w[32 + i] = mma::pack_remainder(a, b, w[i]);
+      }
+      l = fmaf(l, fix, sum0 + sum1);
+      if (v >= 2) {                                          // the products that read this P buffer
+        alive = mbar_wait(&sm.o_done[v & 1], ((v - 2) >> 1) & 1, p.error);
+        if (!__all_sync(0xffffffffu, alive)) { alive = false; break; }
+      }
+      if (v > 0 && __any_sync(0xffffffffu, fix != 1.0f)) {   // the products before have added to O
+        alive = mbar_wait(&sm.o_done[(v - 1) & 1], ((v - 1) >> 1) & 1, p.error);
+        if (!__all_sync(0xffffffffu, alive)) { alive = false; break; }
+        tc_fence_after();
+#pragma unroll 1
+        for (int n = 0; n < R; n += 16) {
+          uint32_t o[16];
+          tmem_ld16(lanes + kLuO + n, o);
+          tmem_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * fix);
+          tmem_st16(lanes + kLuO + n, o);
+        }
+      }
+      tc_fence_after();
+      tmem_st64(lanes + kLuP + (v & 1) * 64, w);
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.p_full[v & 1]);
+    }
+    alive = alive && mbar_wait(&sm.o_done[(visits - 1) & 1], ((visits - 1) >> 1) & 1, p.error);
+    __syncwarp();
+    tc_fence_after();
+    float fold = 1.0f, total = l;
+    if (p.sink != nullptr) {                                 // the sink's term, in the exp2 domain like the others
+      const float s = p.sink[head] * kLuLog2e, high_of = fmaxf(m, s);
+      fold = exp2f(m - high_of);
+      total = fmaf(l, fold, exp2f(s - high_of));
+    }
+    if (row < nrows && alive && (!(total > 0.0f) || total > 3.0e38f)) publish_error(p.error, kAttentionDenominator);
+    float f = total > 0.0f ? fold / total : 0.0f;
+    if (p.gate != nullptr && row < nrows)
+      f *= 1.0f / (1.0f + expf(-__bfloat162float(p.gate[(row0 + row / p.heads) * p.ld_gate + head])));
+    bf16* dst = p.out + (static_cast<long long>(row0) * p.heads + row) * R;
+#pragma unroll 1
+    for (int n = 0; n < R; n += 32) {
+      uint32_t o[32];
+      tmem_ld32(lanes + kLuO + n, o);
+      tmem_wait_ld();
+      if (row >= nrows) continue;                            // (the loads above are the whole warp's)
+      bool finite = true;
+#pragma unroll
+      for (int i = 0; i < 32; ++i) finite = finite && (o[i] & 0x7f800000u) != 0x7f800000u;
+      if (!finite) {
+        const bf16* qr = q_tile + row * R;
+        float acc[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
+        for (int j = first; j <= pos; ++j) {
+          const int slot = slot_of(j);
+          if (slot < 0) continue;
+          const bf16* lr = p.cache + static_cast<long long>(slot) * R;
+          float dot = 0.0f;
+          for (int i = 0; i < R; ++i) dot = fmaf(__bfloat162float(qr[i]), __bfloat162float(lr[i]), dot);
+          const float weight = mma::exp2_fast(fmaf(dot, c, m == -INFINITY ? 0.0f : -m));
+#pragma unroll
+          for (int i = 0; i < 32; ++i) acc[i] = fmaf(weight, __bfloat162float(lr[n + i]), acc[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(acc[i]);
+      }
+#pragma unroll
+      for (int i = 0; i < 32; i += 8)
+        *reinterpret_cast<uint4*>(dst + n + i) =
+            make_uint4(mma::pack(__uint_as_float(o[i]) * f, __uint_as_float(o[i + 1]) * f), mma::pack(__uint_as_float(o[i + 2]) * f, __uint_as_float(o[i + 3]) * f),
+                       mma::pack(__uint_as_float(o[i + 4]) * f, __uint_as_float(o[i + 5]) * f), mma::pack(__uint_as_float(o[i + 6]) * f, __uint_as_float(o[i + 7]) * f));
+    }
+    tc_fence_before();
+  }
+  __syncwarp();
+  __syncthreads();
+  if (warp == 6) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512));
+}
+
+template <int R>
+static int launch_latent_umma(const LatentUmmaArgs& p, unsigned tiles, cudaStream_t s) {
+  const int smem = static_cast<int>(sizeof(LatentUmmaSmem<R>)) + 1024;
+  static bool raised = false;                               // per instance
+  if (!raised) {
+    const cudaError_t e = cudaFuncSetAttribute(latent_attention_umma_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    raised = true;
+  }
+  launch_kernel(latent_attention_umma_kernel<R>, dim3(tiles), dim3(kLuThreads), smem, s, p);
+  PIH_LAUNCH_CHECK();
+  return 0;
+}
+
+}  // namespace pih
+
+using namespace pih;
+
+// bf16; q and out [rows, heads, rank], cache [num_pages, page_size, rank].  PIH_ERR_UNSUPPORTED for other ranks than 64, 128, 192
+// and 256, head counts that do not divide 128, a scale that is not positive, rows that do not begin on 16 bytes.
+extern "C" int pih_latent_attention_tcgen05(const void* q, const void* gate, long long ld_gate, const void* sink, const void* cache,
+                                            const void* block_table, int table_width, const void* positions, const void* cu_q,
+                                            int requests, void* out, int rows, int heads, int rank, int page_size, int num_pages,
+                                            float scale, int window, void* error, void* stream) {
+  if (rows <= 0) return 0;
+  if (heads < 1 || 128 % heads || rank < 64 || rank > 256 || rank % 64 || !(scale > 0.0f) ||
+      ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(cache)) & 15))
+    return PIH_ERR_UNSUPPORTED;
+  LatentUmmaArgs p = {};
+  p.q = static_cast<const __nv_bfloat16*>(q);
+  p.out = static_cast<__nv_bfloat16*>(out);
+  p.gate = static_cast<const __nv_bfloat16*>(gate);
+  p.ld_gate = ld_gate;
+  p.sink = static_cast<const float*>(sink);
+  p.cache = static_cast<const __nv_bfloat16*>(cache);
+  p.block_table = static_cast<const int*>(block_table);
+  p.table_width = table_width;
+  p.positions = static_cast<const int*>(positions);
+  p.cu_q = static_cast<const int*>(cu_q);
+  p.requests = requests, p.heads = heads, p.page_size = page_size, p.num_pages = num_pages, p.window = window;
+  p.scale = scale;
+  p.error = static_cast<uint32_t*>(error);
+  const int tokens = kLuRows / heads;
+  const unsigned tiles = static_cast<unsigned>((rows + tokens - 1) / tokens + requests);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  switch (rank) {
+    case 64: return launch_latent_umma<64>(p, tiles, s);
+    case 128: return launch_latent_umma<128>(p, tiles, s);
+    case 192: return launch_latent_umma<192>(p, tiles, s);
+    default: return launch_latent_umma<256>(p, tiles, s);
+  }
+}

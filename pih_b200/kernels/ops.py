@@ -107,7 +107,7 @@ class CudaOps:
                      "pih_qk_attention_fused", "pih_gemm_tcgen05_pair", "pih_set_attention_side_by_side", "pih_set_skinny_rule",
                      "pih_gemm_simt_batched", "pih_embedding_stream", "pih_rmsnorm_stream", "pih_causal_conv",
                      "pih_gated_delta_rule", "pih_gated_rmsnorm", "pih_rglru_scan", "pih_latent_write",
-                     "pih_latent_attention_generic", "pih_moe_route", "pih_moe_experts", "pih_moe_combine_bf16", "pih_latent_attention_split", "pih_latent_attention_splits", "pih_latent_attention_mma", "pih_batched_gemv",
+                     "pih_latent_attention_generic", "pih_moe_route", "pih_moe_experts", "pih_moe_combine_bf16", "pih_latent_attention_split", "pih_latent_attention_splits", "pih_latent_attention_mma", "pih_latent_attention_tcgen05", "pih_batched_gemv",
                      "pih_stream_cast", "pih_stream_norm_add", "pih_bias_xielu", "pih_add_gated", "pih_retention",
                      "pih_diff_qk_prepare", "pih_diff_attention", "pih_diff_attention_tile_takes", "pih_moe_route_scored",
                      "pih_act_mul", "pih_embed_positions", "pih_hyper_stream", "pih_window_qk_prepare",
@@ -741,6 +741,27 @@ class CudaOps:
     #     8, 256          22.5/34.1  33.7/42.4  42.8/44.3  55.9/51.2  92.3/75.3   130/93    279/172
     #     8, 512          31.0/36.9  52.1/51.4  63.8/63.2  94.3/77.7   163/122    241/178   598/373
     latent_pairs_rows_above = 448
+    latent_tcgen05 = True                  # prompt portions on tcgen05 where that pays; "always", or False: never
+
+    def _latent_on_tcgen05(self, rows: int, heads: int, rank: int, requests: int, window: int, table_keys: int) -> bool:
+        """Whether a portion's latent attention takes the tcgen05 kernel.  There a block walks over all keys of its rows, on
+        mma.sync few rows' keys are cut into parts side by side; so the first is the slower one for a portion of few rows
+        behind a long context.  us, mma.sync / tcgen05, a window of 1024:
+            heads, rank   (past, rows): (0, 65)   (0, 300)   (0, 2048)   (2000, 100)   (2000, 500)   64 of one row and (0, 100)
+            8, 64                     18.9/9.7   15.9/11.0   58.3/27.7    20.3/26.8     36.8/27.2     29.5/31.1
+            16, 128                   24.8/10.1  28.6/12.6  128.3/50.3    30.1/30.2     53.8/30.5     35.0/33.3
+            8, 256                    24.9/12.6  35.0/15.4  148.9/42.3    40.2/39.3     78.8/39.8     58.8/42.5
+            16, 256                   35.7/11.9  52.3/15.6  289.0/68.2    55.8/39.9    103.3/40.7     65.3/42.4
+        What the lengths of the contexts are only the device knows: the two lines below are for the longest that the window
+        and the block table allow."""
+        if self.latent_tcgen05 in (False, "always"):
+            return bool(self.latent_tcgen05)
+        reach = min(table_keys, window) if window > 0 else table_keys
+        waves = -(-(-(-rows * heads // 128) + requests) // 148)
+        here = waves * (3.0 + reach * (0.02 + 6e-5 * rank))
+        there = 14.0 + 0.055 * rank + 5e-8 * rows * heads * reach * rank
+        return here <= there
+
     latent_split = True                    # bf16 attention over a latent: keys cut into parts (False: the in-order kernel)
     batched_library_min_rows = 128         # bf16 batched products of at least this many rows are the library's
 
@@ -994,6 +1015,16 @@ class CudaOps:
             # a row's keys are cut into ``splits`` parts side by side, and each of a block's 8 warps is a part of its own
             # steps of many rows (prompt portions): a block is 4 consecutive rows of a request, which share a tile, or 8
             # of at most 8 heads, two rows of which fill an MMA
+            if T > self.latent_mma_rows_above and self._latent_on_tcgen05(T, heads, rank, step.num_requests, window,
+                                                                          block_table.shape[1] * page_size):
+                # prompt portions: 128 / heads tokens of a request with all their heads a block, nothing to merge
+                rc = self.lib.pih_latent_attention_tcgen05(
+                    _ptr(q), _ptr(gate), c_ll(gate.stride(0) if gate is not None else 0), _ptr(sink), _ptr(cache),
+                    _ptr(block_table), block_table.shape[1], _ptr(step.positions), _ptr(step.cu_q), step.num_requests,
+                    _ptr(out), T, heads, rank, page_size, num_pages, c_float(scale), int(window), self._err(), self._stream())
+                if rc != -2:
+                    self._check(rc, "latent_attention_tcgen05")
+                    return out
             per_block = 1 if T <= self.latent_mma_rows_above else (8 if heads <= 8 and T > self.latent_pairs_rows_above else 4)
             blocks = (T if per_block == 1 else -(-T // per_block) + step.num_requests) * (-(-heads // 16)) * (2 if rank > 256 else 1)
             splits = max(1, min(16, (2 * 148) // max(1, blocks)))

@@ -1,0 +1,67 @@
+"""Latent attention of prompts on tcgen05 against the mma.sync kernel and its merge: sinks, gates, windows, requests that end
+inside a tile, pages that are no power of two, and latents that are not finite."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+PAGE = 24
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from pih_b200.kernels import get_ops
+    return get_ops(torch.device(DEV))
+
+
+def _case(rank, heads, requests, seed):
+    g = torch.Generator(DEV).manual_seed(seed)
+    normal = lambda *s: torch.randn(*s, generator=g, device=DEV).to(torch.bfloat16)
+    width = max(-(-(past + n) // PAGE) for past, n in requests)
+    table = torch.randperm(width * len(requests), generator=torch.Generator().manual_seed(seed)).int().reshape(len(requests), width)
+    cu = [0]
+    for _, n in requests:
+        cu.append(cu[-1] + n)
+    t = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    step = SimpleNamespace(positions=t([past + i for past, n in requests for i in range(n)]), cu_q=t(cu), num_requests=len(requests),
+                           request_of_row=t([r for r, (_, n) in enumerate(requests) for _ in range(n)]))
+    return dict(q=normal(cu[-1], heads, rank), cache=normal(width * len(requests), PAGE, rank) * 0.7, block_table=table.to(DEV),
+                step=step, scale=rank ** -0.5), normal
+
+
+@pytest.mark.parametrize("rank,heads", [(64, 1), (64, 128), (128, 2), (192, 32), (256, 8), (256, 16)])
+@pytest.mark.parametrize("requests", [[(0, 65)], [(130, 129)], [(0, 40), (700, 1), (63, 33)], [(1000, 257)]])
+@pytest.mark.parametrize("window", [0, 1, 100])
+def test_against_mma_sync(ops, rank, heads, requests, window):
+    case, normal = _case(rank, heads, requests, seed=rank + heads)
+    rows = case["q"].shape[0]
+    options = dict(gate=normal(rows, heads), sink=normal(heads).float(), window=window)
+    try:
+        ops.latent_tcgen05 = "always"
+        got = ops.latent_attention(**case, **options)
+        ops.latent_tcgen05 = False
+        want = ops.latent_attention(**case, **options)
+    finally:
+        del ops.latent_tcgen05
+    ops.check_errors()
+    # there the weights are rounded to 8 bits (2^-9 of a term, in random directions), both round the output once
+    worst = float(((got.double() - want.double()).norm(dim=-1) / want.double().norm(dim=-1)).max())
+    assert worst < 1.5e-2, worst
+
+
+def test_a_latent_that_is_not_finite_reaches_the_rows_that_see_it_alone(ops, monkeypatch):
+    monkeypatch.setattr(ops, "latent_tcgen05", "always", raising=False)
+    rank, heads, n, at, window = 256, 8, 200, 100, 40
+    case, _ = _case(rank, heads, [(0, n)], seed=5)
+    place = case["block_table"][0, at // PAGE].long(), at % PAGE
+    case["cache"][place] = 0
+    want = ops.latent_attention(**case, gate=None, sink=None, window=window).float()
+    case["cache"][place[0], place[1], 7] = float("inf")
+    got = ops.latent_attention(**case, gate=None, sink=None, window=window).float()
+    ops.clear_errors()
+    sees = torch.zeros(n, dtype=torch.bool, device=DEV)
+    sees[at:at + window] = True
+    assert torch.isfinite(got[~sees]).all()
+    torch.testing.assert_close(got[~sees], want[~sees], rtol=2.0 ** -7, atol=2.0 ** -12)
